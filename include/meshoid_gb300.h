@@ -225,6 +225,11 @@ int mg_hsml_solve(const float *d2, int64_t nq, int32_t k, int32_t dim, float *hs
 int mg_neighbor_dist(const mg_cells *cells, const int32_t *queries, int64_t nq, const int32_t *ngb,
                      int32_t k, int64_t *ngb_particles, double *dist, void *stream);
 
+/* mg_neighbor_dist with each query's row written at row out_rows[q] of both
+ * outputs (NULL: row q). */
+int mg_neighbor_lists(const mg_cells *cells, const int32_t *queries, int64_t nq, const int32_t *ngb,
+                      int32_t k, const int32_t *out_rows, int64_t *ngb_particles, double *dist, void *stream);
+
 /* ---- fields and derivatives --------------------------------------------- */
 /* Gather f (n, nf) FP64 particle order into slot order as an FP32 pair
  * hi + lo = f (to ~48 bits).  Both outputs are (n, nfp) row-major with

@@ -100,6 +100,7 @@ SIGNATURES = {
     "mg_knn_hsml": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i64, c_i32, c_vp, c_f32, c_i32, c_i32, c_vp,
                             c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "mg_neighbor_dist": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i64, c_vp, c_i32, c_vp, c_vp, c_vp]),
+    "mg_neighbor_lists": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i64, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp]),
     "mg_load_fields": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i32, c_vp, c_vp, c_vp]),
     "mg_load_fields3": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i32, c_vp, c_vp, c_vp, c_vp]),
     "mg_hsml_polish": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i64, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp]),

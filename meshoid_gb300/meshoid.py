@@ -406,14 +406,9 @@ class Meshoid:
         nq, k = self._ngb_slots.shape
         idx = torch.empty((nq, k), dtype=torch.int64, device=self.device)
         dist = torch.empty((nq, k), dtype=torch.float64, device=self.device)
-        check(self._lib.mg_neighbor_dist(self._cells, ptr(self._queries), nq, ptr(self._ngb_slots), k,
-                                         ptr(idx), ptr(dist), _stream()), "mg_neighbor_dist")
-        rows = self._out_rows.long()
-        ui = torch.empty_like(idx)
-        ud = torch.empty_like(dist)
-        ui[rows] = idx
-        ud[rows] = dist
-        self._ngb_user, self._ngbdist_user = ui, ud
+        check(self._lib.mg_neighbor_lists(self._cells, ptr(self._queries), nq, ptr(self._ngb_slots), k,
+                                          ptr(self._out_rows), ptr(idx), ptr(dist), _stream()), "mg_neighbor_lists")
+        self._ngb_user, self._ngbdist_user = idx, dist
 
     def _kth_distance(self):
         """Distance to the k-th (farthest) neighbour of each query, internal query order (FP64)."""
