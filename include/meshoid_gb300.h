@@ -164,8 +164,9 @@ size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k);
  * h solving norm * sum_j W(d_j / h) = k over those neighbours.
  *   seed_h: nq FP32 first guesses of h; the first search radius is
  *           radius_factor * seed_h.  A query whose radius holds fewer than k
- *           particles (or too many) is re-queued with a corrected radius, up to
- *           max_passes passes.
+ *           particles (or too many) is searched again with a corrected
+ *           radius, up to 4 max_passes times (max_passes 1: once; k > 32: in
+ *           up to max_passes passes).
  *   level_bias: 0 or 1 -- the searched cells have side >= R / 2^level_bias
  *           (finer cells: fewer candidates, more cell lookups).
  *   ngb:    nq * k slots, unordered within a row (the set is exact: the k
@@ -177,11 +178,13 @@ size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k);
  *           with mg_hsml_polish).  hsml alone is good to ~1e-7.
  *           qstatus: nq MG_Q_* bits.
  *   stats:  16 int64 device counters, accumulated (the caller zeroes them):
- *           [0] passes after the first, [1] candidates scanned (warp passes)
- *           or staged (first pass, per query it serves), [2] retries,
- *           [3] FP64 band re-decisions, [4] unresolved, [5] Newton steps,
- *           [6..8] retries for too few / too many / band outside the radius,
- *           [9] queries handed to the block-wide path (scan list > 2048).
+ *           [0] most searches any query took after its first in the warp
+ *           path (k > 32: passes after the first), [1] candidates scanned (warp path) or staged (first pass,
+ *           per query it serves), [2] retries, [3] FP64 band re-decisions,
+ *           [4] unresolved, [5] Newton steps, [6..8] retries for too few /
+ *           too many / band outside the radius, [9] scan lists narrowed
+ *           before the scan, or for k > 32 handed to a block (crowded: a
+ *           sparse query beside a dense clump).
  * Replaces tree.query + HsmlIter (src/meshoid/Meshoid.py:157,165;
  * src/meshoid/kernel_density.py:15-56). */
 int mg_knn_hsml(const mg_cells *cells, const int32_t *queries, int64_t nq, int32_t k,
@@ -191,19 +194,13 @@ int mg_knn_hsml(const mg_cells *cells, const int32_t *queries, int64_t nq, int32
                 size_t workspace_bytes, void *stream);
 /* First pass of mg_knn_hsml: 1 (default) runs it one thread per query over
  * candidates staged once per block of 128 consecutive queries, the queries it
- * cannot decide exactly going on to the warp-per-query passes; 0 runs every
- * pass warp per query.  Both give the same neighbour sets and distances.
+ * cannot decide exactly going on to the warp-per-query path; 0 runs every
+ * query there.  Both give the same neighbour sets and distances.
  * Process-wide; returns the previous setting. */
 int mg_knn_set_group_pass(int32_t enabled);
-/* Passes after the first of mg_knn_hsml: 1 runs them in one cooperative
- * launch that drains the device-side work queue (the warp path, a grid-wide
- * barrier, the block-wide path for crowded queries, a barrier; it ends when a
- * pass starts on an empty queue); 0 (the default) launches the kernels of
- * every pass from the host (max_passes of them, most on an empty queue).
- * Both give the same neighbour sets, distances and h; measured on a GB300
- * the cooperative launch is no faster on one snapshot (as fast on a Plummer
- * sphere, 3% slower on a clump mixture) and keeps concurrent streams from
- * overlapping.  Process-wide; returns the previous setting. */
+/* Kept for its callers: the warp path of mg_knn_hsml is one launch of
+ * persistent warps whatever this is set to.  Process-wide; returns the
+ * previous setting (0 at start). */
 int mg_knn_set_persistent_passes(int32_t enabled);
 /* Smoothing lengths, densities and volumes in output-row order
  * (src/meshoid/Meshoid.py:169-170): for query q, row r = out_rows[q] (or q),

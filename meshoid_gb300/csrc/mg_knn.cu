@@ -8,21 +8,19 @@
 // staged once per block of 128 consecutive queries; it accepts a query only
 // when an error bound proves its set exact, and queues the rest.
 //
-// Search, warp passes (k_knn_hsml; every pass for periodic boxes or k > 32):
+// Search, warp path (k_knn_hsml; every query for periodic boxes or k > 32):
 // the query's radius R comes from a seed or the queue.  The level L with cell
 // side s_L >= R (or R / 2) is chosen, the level-L cells that meet the sphere
 // of radius R are looked up (dense table for L <= grid_level, refinement
-// tables or a binary search of the Morton keys below), and every particle of
-// those cells with FP32 d^2 <= R^2 is appended to a per-warp shared-memory
-// buffer.  Fewer than k hits, or more than the buffer holds, re-queues the
-// query with a corrected radius (work queue over passes).  The k smallest are
+// tables or a binary search of the Morton keys below), a list of too many
+// particles is narrowed by splitting its cells (narrow_list), and every
+// particle of those cells with FP32 d^2 <= R^2 is appended to a per-warp
+// shared-memory buffer.  Fewer than k hits, or more than the buffer holds, and
+// the warp searches again with a corrected radius.  The k smallest are
 // picked by a 32-bucket histogram in (d/R)^dim; entries within 1e-5
 // (relative, in d^2) of the k-th distance are re-decided with exact FP64
 // distances and the particle index, so the set equals the k smallest by
-// (FP64 d^2, index).  A query whose cells hold more than 2048 particles (a
-// sparse query next to a dense clump) is handed with its cell list to a
-// block-wide kernel, so that no warp scans a long list alone while the grid
-// waits for it.
+// (FP64 d^2, index).
 //
 // h: norm * sum_j W(d_j/h) = k (norm = 32/3, 40/7, 8/3 in 3/2/1-D), solved by
 // bracketed Newton (bisection fallback), one thread per query, on the k FP32
@@ -33,16 +31,12 @@
 #include <atomic>
 #include <cfloat>
 
-#include <cooperative_groups.h>
-
 #include "mg_common.cuh"
 #include "mg_grad2.cuh"
 #include "mg_hsml.cuh"
 #include "mg_refine.cuh"
 
 namespace mg {
-
-namespace cg = cooperative_groups;
 
 constexpr int kKnnWarps = 8;     // warps per block
 constexpr float kBandEps = 1e-5f;
@@ -60,29 +54,26 @@ constexpr float kBandEps = 1e-5f;
 #define MG_KNN_MINBLOCKS 4
 #endif
 constexpr int kKnnMinBlocks = MG_KNN_MINBLOCKS;  // resident blocks per SM the register budget is cut for
-#ifndef MG_KNN_CHUNK
-#define MG_KNN_CHUNK 32
-#endif
-#ifndef MG_KNN_SPLIT
-#define MG_KNN_SPLIT 192
-#endif
-constexpr int kChunk = MG_KNN_CHUNK;  // consecutive queries per warp on the first pass
-constexpr int kSplit = MG_KNN_SPLIT;  // cells holding more particles than this are split when they straddle the sphere
 constexpr int kList = 128;       // scan-list capacity per warp
-constexpr int kScanLimit = 1 << 20;  // scan-list particles above which a first radius is halved unscanned
-// Queries per run dealt to a warp of the warp passes in turn (0: one
-// contiguous run per warp).  The queue's cost is uneven (the slowest warp of
-// a contiguous split took 1.8x the mean), and balance pays more than the
-// cell-box reuse of long runs: search + h at 2^22 (Plummer / clump mixture)
-// 10.83 / 19.82 ms with contiguous runs, 10.70 / 19.23 with runs of 4,
-// 10.68 / 18.38 with single queries.
-#ifndef MG_KNN_WCHUNK
-#define MG_KNN_WCHUNK 1
+constexpr int kScanLimit = 1 << 20;  // scan-list particles above which a first radius is cut unscanned
+// Scan-list particles above which the list is narrowed (narrow_list) before it
+// is scanned: about three times what a sphere with a buffer-full of
+// neighbours lists.
+#ifndef MG_KNN_NARROW
+#define MG_KNN_NARROW 640
 #endif
-#ifndef MG_KNN_HEAVY
-#define MG_KNN_HEAVY 2048
-#endif
-constexpr int kHeavy = MG_KNN_HEAVY;  // scan-list particles above which a query goes to the block-wide path
+constexpr int kNarrow = MG_KNN_NARROW;
+constexpr int kNarrowCell = 48;  // cells of up to this many particles are not split
+// Queries taken from the common counter at a time: one from the queue, whose
+// cost is uneven (2^22 clump mixture, searching: 18.4 ms one at a time, 19.2
+// in runs of four), a run of consecutive queries when the warp path serves
+// them all, so that a warp reuses its cell box.
+constexpr unsigned kRun = 8;
+
+// Passes over the queue for k > 32 (k_knn_pass, k_knn_heavy)
+constexpr int kChunk = 32;     // consecutive queries per warp on the first pass
+constexpr int kSplit = 192;    // cells holding more particles than this are split when they straddle the sphere
+constexpr int kHeavy = 2048;   // scan-list particles above which a query goes to the block-wide path
 constexpr int kHeavyItem = 2 * kList + 4;  // int32 words per queued heavy query: qi, nlist, pa[], off[]
 constexpr int kHeavyThreads = 256;
 constexpr int kHeavyBins = 1024;
@@ -108,18 +99,23 @@ struct KnnArgs {
     const float *seed_h;
     float radius_factor;
     float *radius;
-    float *rlo;  // largest radius seen with fewer than k particles (0: none)
-    float *rhi;  // smallest radius seen with too many particles to scan (0: none)
     int32_t *ngb;
     float *hsml;
     int32_t *qstatus;
-    const int32_t *qin;          // nullptr on the first pass
+    const int32_t *qin;          // queries of the warp path (nullptr: all of them)
     const int32_t *qin_count;
-    int32_t *qout;
+    unsigned *next;              // next query of the warp path to take
+    int32_t *qout;               // queries that the first pass leaves to the warp path
     int32_t *qout_count;
     int64_t *stats;
-    int last_pass;
+    int max_tries;   // radii searched per query
     int level_bias;  // search cells of side s with s >= R / 2^level_bias
+};
+
+struct KnnPassArgs : KnnArgs {
+    float *rlo;  // largest radius seen with fewer than k particles (0: none)
+    float *rhi;  // smallest radius seen with too many particles to scan (0: none)
+    int last_pass;
     int32_t *heavy;        // heavy-query items of this pass (kHeavyItem words each)
     int32_t *heavy_count;  // items queued this pass (may exceed heavy_cap: the excess was not queued)
     int32_t *heavy_next;   // next item to take (block-wide path)
@@ -200,12 +196,13 @@ struct KnnSmem {
     float sel[32 * KPL];            // d^2 of the selected neighbours
     uint32_t ca[kList], cb[kList];  // cached box: cell ranges by box index
     uint32_t pa[kList], pb[kList];  // scan list of the current query
-    uint64_t pc[kList];             // scan-list cell: level | x << 5 | y << 24 | z << 43
+    uint64_t pc[kList];             // scan-list cell: level | x << 5 | y << 24 | z << 43 (periodic: x + 2^level, ..)
     uint32_t off[kList + 1];        // scan-list prefix offsets
 };
 
 struct WarpStats {
     int64_t cand = 0, retry = 0, band = 0, unres = 0, newton = 0, heavy = 0;
+    int tries = 0;
     int64_t reason[3] = {0, 0, 0};
     int64_t phase[6] = {0, 0, 0, 0, 0, 0};
 };
@@ -444,70 +441,200 @@ __device__ KNN_LAZY_INLINE void lazy_hist_init(SM &S, float invR2) {
     __syncwarp();
 }
 
-// Rare path (out of line): entries of the scan-list chunk starting at i0 that
-// hold more than kSplit particles and straddle the sphere are replaced by their
-// non-empty children that meet it (open 3-D boxes; children of a level-l cell
-// are consecutive Morton codes, so 7 binary searches inside the parent's range
-// give all 8 ranges).  Returns the new list length.
-template <class SM>
-__device__ __noinline__ int split_chunk(SM &S, int i0, int nlist, float ux0, float uy0, float uz0, float Rs, float rc,
-                                        int L, const uint64_t *__restrict__ keys) {
+// Rare path (out of line): a scan list of too many particles (a sparse query
+// beside a dense clump, a first radius far too large) is narrowed before it is
+// scanned.  Each round (1) bounds the k-th distance from above: the far
+// corners of the listed cells, binned in 32 shells between the nearest of them
+// and the radius (a clump seen from afar fills few shells of the whole radius),
+// and the first shell by which cells of at least k particles lie inside it
+// entirely; (2) drops the cells beyond that radius; (3) splits the larger
+// cells into their non-empty children, four cells at a time, one child per lane
+// (table lookups down to the refinement tables' leaves), the nearest first: a
+// tighter bound drops most of the others unsplit, whereas splitting them in
+// list order filled the list with cells of the clump's whole near face (one
+// query of 2^24 clumped particles then took 28 ms).  The list stays complete
+// for the radius it returns, which holds at least k particles.
+// Handing such a query with its whole list to a block of 256 threads, which
+// read every listed particle at least twice, took 4.9 of the 9.5 ms of 10^6
+// Plummer particles with learned first radii, and 19.5 ms of 2^24 clumped
+// ones.  Lengths in sides of the level-L cells; m0: rounding margin.
+template <int DIM, class SM>
+__device__ __noinline__ int narrow_list(SM &S, const KnnArgs &a, int32_t p, int nlist, int target, int L, float ux,
+                                        float uy, float uz, int full, float scale, float m0, float &Rl) {
+    const bool periodic = a.periodic;
+    const int k = a.k;
     const int lane = threadIdx.x & 31;
-    const int i = i0 + lane;
-    bool split = false;
-    if (i < nlist && S.pb[i] - S.pa[i] > (uint32_t)kSplit) {
-        const uint64_t pc = S.pc[i];
+    const float half_box = 0.5f * (float)(1u << L);
+    auto corners = [&](uint64_t pc, float &near2, float &far2) {
         const int lv = (int)(pc & 31u);
-        if (lv < kMaxLevel) {
-            const float f = exp2f((float)(lv - L));
-            const float x0 = (float)((pc >> 5) & 0x7ffffu), y0 = (float)((pc >> 24) & 0x7ffffu),
-                        z0 = (float)((pc >> 43) & 0x7ffffu);
-            const float ux = ux0 * f, uy = uy0 * f, uz = uz0 * f;
-            const float fx = fmaxf(fabsf(ux - x0), fabsf(ux - x0 - 1.0f));
-            const float fy = fmaxf(fabsf(uy - y0), fabsf(uy - y0 - 1.0f));
-            const float fz = fmaxf(fabsf(uz - z0), fabsf(uz - z0 - 1.0f));
-            const float rin = Rs * f * (1.0f - 1e-5f);
-            split = fx * fx + fy * fy + fz * fz > rin * rin;  // not entirely inside
-        }
-    }
-    unsigned sm = __ballot_sync(0xffffffffu, split);
-    while (sm) {
-        const int j = __ffs(sm) - 1;
-        sm &= sm - 1;
-        const int idx = i0 + j;
-        const uint32_t A = S.pa[idx], B = S.pb[idx];
-        const uint64_t pc = S.pc[idx];
-        const int lv = (int)(pc & 31u) + 1;
-        const uint32_t x0 = (uint32_t)((pc >> 5) & 0x7ffffu) * 2u, y0 = (uint32_t)((pc >> 24) & 0x7ffffu) * 2u,
-                       z0 = (uint32_t)((pc >> 43) & 0x7ffffu) * 2u;
-        const int ch = lane & 7;
-        const uint32_t cx = x0 + (ch & 1), cy = y0 + ((ch >> 1) & 1), cz = z0 + (ch >> 2);
-        const uint64_t code = morton3(cx, cy, cz);
-        uint32_t lo = A;
-        if (lane >= 1 && lane < 8) lo = lower_bound_prefix(keys, A, B, code, 3 * (kKeyBits - lv));
-        uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
-        if (ch == 7) hi = B;
-        bool keep = false;
-        if (lane < 8 && hi > lo) {
-            const float f = exp2f((float)(lv - L));
-            const float ux = ux0 * f, uy = uy0 * f, uz = uz0 * f, rr = rc * f;
-            const float dx = fmaxf(0.0f, fmaxf((float)cx - ux, ux - (float)(cx + 1)));
-            const float dy = fmaxf(0.0f, fmaxf((float)cy - uy, uy - (float)(cy + 1)));
-            const float dz = fmaxf(0.0f, fmaxf((float)cz - uz, uz - (float)(cz + 1)));
-            keep = dx * dx + dy * dy + dz * dz <= rr * rr;
-        }
-        const unsigned km = __ballot_sync(0xffffffffu, keep);
-        if (nlist + __popc(km) <= kList) {
-            const int pos = nlist + __popc(km & ((1u << lane) - 1u));
-            if (keep) {
-                S.pa[pos] = lo;
-                S.pb[pos] = hi;
-                S.pc[pos] = (uint64_t)lv | ((uint64_t)cx << 5) | ((uint64_t)cy << 24) | ((uint64_t)cz << 43);
+        const float f = exp2f((float)(L - lv));
+        const int off = periodic ? 1 << lv : 0;
+        const float u[3] = {ux, uy, uz};
+        near2 = far2 = 0.0f;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            const float x0 = (float)((int)((pc >> (5 + 19 * d)) & 0x7ffffu) - off) * f, x1 = x0 + f;
+            float nr = fmaxf(0.0f, fmaxf(x0 - u[d], u[d] - x1));
+            float fa = fmaxf(fabsf(u[d] - x0), fabsf(u[d] - x1));
+            if (full >> d & 1) {  // every cell of the axis is listed once, unwrapped
+                nr = 0.0f;
+                fa = fminf(fa, half_box);
             }
-            nlist += __popc(km);
-            if (lane == 0) S.pb[idx] = S.pa[idx];  // parent replaced by its children
+            near2 += nr * nr;
+            far2 += fa * fa;
+        }
+    };
+    for (int round = 0; round < 32; ++round) {
+        S.hist[lane] = 0;
+        float least = Rl;
+        for (int i = lane; i < nlist; i += 32) {
+            float near2, far2;
+            corners(S.pc[i], near2, far2);
+            if (S.pb[i] > S.pa[i]) least = fminf(least, sqrtf(far2) * 1.000001f + m0);
+        }
+        least = warp_min(least);
+        const float width = (Rl - least) * (1.0f / 32.0f), bscale = 1.0f / fmaxf(width, 1e-30f);
+        for (int i = lane; i < nlist; i += 32) {
+            const int c = (int)(S.pb[i] - S.pa[i]);
+            float near2, far2;
+            corners(S.pc[i], near2, far2);
+            const float t = (sqrtf(far2) * 1.000001f + m0 - least) * bscale;
+            if (c > 0 && t < 32.0f) atomicAdd(&S.hist[max(0, (int)t)], c);
         }
         __syncwarp();
+        const int cum = warp_incl_scan(S.hist[lane]);
+        const unsigned reach = __ballot_sync(0xffffffffu, cum >= k);
+        if (reach) Rl = fminf(Rl, (least + width * (float)__ffs(reach)) * 1.000001f);
+        // keep what meets the sphere, find what to split
+        const float rc = Rl * (1.0f + 1e-5f) + m0;
+        int w = 0, total = 0;
+        for (int i0 = 0; i0 < nlist; i0 += 32) {
+            const int i = i0 + lane;
+            const uint32_t ca = i < nlist ? S.pa[i] : 0u, cb = i < nlist ? S.pb[i] : 0u;
+            const uint64_t pc = i < nlist ? S.pc[i] : 0ull;
+            float near2 = 0.0f, far2;
+            if (cb > ca) corners(pc, near2, far2);
+            const bool keep = cb > ca && near2 <= rc * rc;
+            const unsigned m = __ballot_sync(0xffffffffu, keep);  // (also: the chunk is read before it is rewritten)
+            if (keep) {
+                const int pos = w + __popc(m & ((1u << lane) - 1u));
+                S.pa[pos] = ca;
+                S.pb[pos] = cb;
+                S.pc[pos] = pc;
+            }
+            w += __popc(m);
+            total += __reduce_add_sync(0xffffffffu, keep ? (int)(cb - ca) : 0);
+            __syncwarp();
+        }
+        nlist = w;
+        if (total <= target) break;
+        // entries lane, lane + 32, .. that may be split, by distance
+        unsigned key[kList / 32];
+#pragma unroll
+        for (int c = 0; c < kList / 32; ++c) {
+            const int i = lane + 32 * c;
+            key[c] = 0xffffffffu;
+            if (i < nlist && (int)(S.pb[i] - S.pa[i]) > kNarrowCell) {
+                float near2, far2;
+                corners(S.pc[i], near2, far2);
+                if ((int)(S.pc[i] & 31u) < (periodic ? kMaxLevel - 1 : kMaxLevel))
+                    key[c] = (__float_as_uint(near2) & ~(unsigned)(kList - 1)) | (unsigned)i;
+            }
+        }
+        bool any = false;
+        for (int step = 0; step < 4; ++step) {
+            // the four nearest, eight lanes each
+            int mine = -1, n = 0;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                unsigned best = key[0];
+#pragma unroll
+                for (int c = 1; c < kList / 32; ++c) best = min(best, key[c]);
+                best = __reduce_min_sync(0xffffffffu, best);
+                if (best == 0xffffffffu) continue;
+                ++n;
+                if (lane >> 3 == g) mine = (int)(best & (unsigned)(kList - 1));
+#pragma unroll
+                for (int c = 0; c < kList / 32; ++c)
+                    if (key[c] == best) key[c] = 0xffffffffu;
+            }
+            if (n == 0) break;
+            uint32_t ca = 0, cb = 0;
+            uint64_t child = 0;
+            if (mine >= 0) {
+                const uint64_t pc = S.pc[mine];
+                const int lv = (int)(pc & 31u) + 1;
+                const uint64_t x = 2 * ((pc >> 5) & 0x7ffffu) + (lane & 1),
+                               y = 2 * ((pc >> 24) & 0x7ffffu) + ((lane >> 1) & 1),
+                               z = 2 * ((pc >> 43) & 0x7ffffu) + ((lane >> 2) & 1);
+                const uint32_t wrap = (1u << lv) - 1u;
+                child = (uint64_t)lv | (x << 5) | (y << 24) | (z << 43);
+                cell_lookup(a.ci, lv, morton3((uint32_t)x & wrap, (uint32_t)y & wrap, (uint32_t)z & wrap), ca, cb);
+            }
+            float near2 = 0.0f, far2;
+            if (cb > ca) corners(child, near2, far2);
+            const bool keep = cb > ca && near2 <= rc * rc;
+            const unsigned km = __ballot_sync(0xffffffffu, keep);
+            // a cell's first child takes its place, the others are appended; a cell
+            // whose children do not fit stays as it is
+            int add = 0, first = -1;  // this group's first appended entry
+            unsigned done = 0u;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int more = max(0, __popc(km >> (8 * g) & 0xffu) - 1);
+                if (g < n && nlist + add + more <= kList) {
+                    if (lane >> 3 == g) first = nlist + add;
+                    done |= 0xffu << (8 * g);
+                    add += more;
+                }
+            }
+            if (!done) break;
+            any = true;
+            if (first >= 0) {
+                const unsigned mk = km >> (lane & 24) & 0xffu;
+                const int r = __popc(mk & ((1u << (lane & 7)) - 1u));
+                const int pos = r == 0 ? mine : first + r - 1;
+                if (keep) {
+                    S.pa[pos] = ca;
+                    S.pb[pos] = cb;
+                    S.pc[pos] = child;
+                } else if (mk == 0u && (lane & 7) == 0) {
+                    S.pb[mine] = S.pa[mine];
+                }
+            }
+            nlist += add;
+            __syncwarp();
+        }
+        if (!any) {
+            // no cell fits (or none is left to split): the bound from the particles
+            // of the small cells themselves
+            const float4 h0 = a.hi[p], l0 = a.lo[p];
+            float least = Rl;
+            S.hist[lane] = 0;
+            for (int i = lane; i < nlist; i += 32) {
+                float near2, far2;
+                corners(S.pc[i], near2, far2);
+                if (S.pb[i] - S.pa[i] <= (uint32_t)kNarrowCell) least = fminf(least, sqrtf(near2));
+            }
+            least = warp_min(least);
+            const float width = (Rl - least) * (1.0f / 32.0f), bscale = 1.0f / fmaxf(width, 1e-30f);
+            __syncwarp();
+            for (int i = 0; i < nlist; ++i) {
+                const uint32_t ca = S.pa[i], cb = S.pb[i];
+                if (cb - ca > (uint32_t)kNarrowCell) continue;
+                for (uint32_t t = ca + lane; t < cb; t += 32) {
+                    const float d = sqrtf(cand_d2(a, h0, l0, t)) * scale * 1.00001f;
+                    const float x = (d - least) * bscale;
+                    if (x < 32.0f) atomicAdd(&S.hist[max(0, (int)x)], 1);
+                }
+            }
+            __syncwarp();
+            const unsigned found = __ballot_sync(0xffffffffu, warp_incl_scan(S.hist[lane]) >= k);
+            const float Rn = found ? (least + width * (float)__ffs(found)) * 1.00001f : Rl;
+            __syncwarp();
+            if (!(Rn < 0.9995f * Rl)) break;
+            Rl = Rn;
+        }
     }
     return nlist;
 }
@@ -604,56 +731,117 @@ __device__ KNN_SELECT_INLINE void finish_row(SM &S, int cnt, float T, int k, int
     }
 }
 
+// ---- k > 32: passes over a queue -------------------------------------------------
+// For k > 32 h is solved in FP32 from the row's distances in the row's order,
+// so that the order of a row, which follows from how its query was searched,
+// shows in h and the density at ~3e-8.  These rows keep the search that
+// produced them so far, and with it every bit of their results: a pass of
+// warps over the queue (k_knn_pass), then a block per crowded query
+// (k_knn_heavy), undecided queries queued for the next pass.  For k <= 32 h is
+// solved in float-float, where the order does not show above 1e-13, and
+// k_knn_hsml decides every query in place.
+// Rare path (out of line): entries of the scan-list chunk starting at i0 that
+// hold more than kSplit particles and straddle the sphere are replaced by their
+// non-empty children that meet it (open 3-D boxes; children of a level-l cell
+// are consecutive Morton codes, so 7 binary searches inside the parent's range
+// give all 8 ranges).  Returns the new list length.
+template <class SM>
+__device__ __noinline__ int split_chunk(SM &S, int i0, int nlist, float ux0, float uy0, float uz0, float Rs, float rc,
+                                        int L, const uint64_t *__restrict__ keys) {
+    const int lane = threadIdx.x & 31;
+    const int i = i0 + lane;
+    bool split = false;
+    if (i < nlist && S.pb[i] - S.pa[i] > (uint32_t)kSplit) {
+        const uint64_t pc = S.pc[i];
+        const int lv = (int)(pc & 31u);
+        if (lv < kMaxLevel) {
+            const float f = exp2f((float)(lv - L));
+            const float x0 = (float)((pc >> 5) & 0x7ffffu), y0 = (float)((pc >> 24) & 0x7ffffu),
+                        z0 = (float)((pc >> 43) & 0x7ffffu);
+            const float ux = ux0 * f, uy = uy0 * f, uz = uz0 * f;
+            const float fx = fmaxf(fabsf(ux - x0), fabsf(ux - x0 - 1.0f));
+            const float fy = fmaxf(fabsf(uy - y0), fabsf(uy - y0 - 1.0f));
+            const float fz = fmaxf(fabsf(uz - z0), fabsf(uz - z0 - 1.0f));
+            const float rin = Rs * f * (1.0f - 1e-5f);
+            split = fx * fx + fy * fy + fz * fz > rin * rin;  // not entirely inside
+        }
+    }
+    unsigned sm = __ballot_sync(0xffffffffu, split);
+    while (sm) {
+        const int j = __ffs(sm) - 1;
+        sm &= sm - 1;
+        const int idx = i0 + j;
+        const uint32_t A = S.pa[idx], B = S.pb[idx];
+        const uint64_t pc = S.pc[idx];
+        const int lv = (int)(pc & 31u) + 1;
+        const uint32_t x0 = (uint32_t)((pc >> 5) & 0x7ffffu) * 2u, y0 = (uint32_t)((pc >> 24) & 0x7ffffu) * 2u,
+                       z0 = (uint32_t)((pc >> 43) & 0x7ffffu) * 2u;
+        const int ch = lane & 7;
+        const uint32_t cx = x0 + (ch & 1), cy = y0 + ((ch >> 1) & 1), cz = z0 + (ch >> 2);
+        const uint64_t code = morton3(cx, cy, cz);
+        uint32_t lo = A;
+        if (lane >= 1 && lane < 8) lo = lower_bound_prefix(keys, A, B, code, 3 * (kKeyBits - lv));
+        uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
+        if (ch == 7) hi = B;
+        bool keep = false;
+        if (lane < 8 && hi > lo) {
+            const float f = exp2f((float)(lv - L));
+            const float ux = ux0 * f, uy = uy0 * f, uz = uz0 * f, rr = rc * f;
+            const float dx = fmaxf(0.0f, fmaxf((float)cx - ux, ux - (float)(cx + 1)));
+            const float dy = fmaxf(0.0f, fmaxf((float)cy - uy, uy - (float)(cy + 1)));
+            const float dz = fmaxf(0.0f, fmaxf((float)cz - uz, uz - (float)(cz + 1)));
+            keep = dx * dx + dy * dy + dz * dz <= rr * rr;
+        }
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        if (nlist + __popc(km) <= kList) {
+            const int pos = nlist + __popc(km & ((1u << lane) - 1u));
+            if (keep) {
+                S.pa[pos] = lo;
+                S.pb[pos] = hi;
+                S.pc[pos] = (uint64_t)lv | ((uint64_t)cx << 5) | ((uint64_t)cy << 24) | ((uint64_t)cz << 43);
+            }
+            nlist += __popc(km);
+            if (lane == 0) S.pb[idx] = S.pa[idx];  // parent replaced by its children
+        }
+        __syncwarp();
+    }
+    return nlist;
+}
+
 template <int DIM, int KPL>
-__device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *knn_smem) {
+__global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_pass(const __grid_constant__ KnnPassArgs a) {
     using SM = KnnSmem<KPL>;
     constexpr int kKnnCap = SM::kCap;
+    extern __shared__ __align__(16) unsigned char knn_smem[];
     SM &S = reinterpret_cast<SM *>(knn_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t gwarp = (int64_t)blockIdx.x * kKnnWarps + wib;
     const int64_t nwarps = (int64_t)gridDim.x * kKnnWarps;
-    // the queue, radii and brackets of this pass were written by other blocks
-    // of an earlier pass (of the same launch, for the cooperative passes): read
-    // at L2 (__ldcg), never from a stale L1 line
-    const int64_t count = a.qin ? (int64_t)__ldcg(a.qin_count) : a.nq;
+    const int64_t count = a.qin ? (int64_t)*a.qin_count : a.nq;
     const Frame fr = load_frame(a.frame);
     const float side = (float)fr.side;
     const float half_side = 0.5f * side;
     const int k = a.k;
 
     WarpStats st;
-#ifdef MG_KNN_PROFILE
-    const long long t_warp0 = clock64();
-#endif
     int32_t my_retry = -1;  // lane i holds the i-th pending retry of this warp
     int n_retry = 0;
 
-    // Each warp takes runs of MG_KNN_WCHUNK queries dealt to the warps in
-    // turn (the slow regions of the queue spread over the warps), or with 0
-    // one contiguous run; a warp reuses the cell-box ranges of its previous
-    // query when the next one needs the same box (consecutive queries are
-    // neighbours in Morton order).
+    // Queries are dealt to the warps in turn (the queue's cost is uneven); a
+    // warp reuses the cell-box ranges of its previous query when the next one
+    // needs the same box.
     int cL = -1, cmin_c[3] = {0, 0, 0}, cnum_c[3] = {0, 0, 0};  // cached box
-#if MG_KNN_WCHUNK > 0
-    for (int64_t c0 = gwarp * MG_KNN_WCHUNK; c0 < count; c0 += nwarps * MG_KNN_WCHUNK)
-    for (int64_t item = c0, item1 = min(count, c0 + (int64_t)MG_KNN_WCHUNK); item < item1; ++item) {
-#else
-    const int64_t per_warp = (count + nwarps - 1) / nwarps;
-    const int64_t item0 = gwarp * per_warp;
-    const int64_t item1 = min(count, item0 + per_warp);
-    for (int64_t item = item0; item < item1; ++item) {
-#endif
-        KNN_TICK(t_a);
-        const int32_t qi = a.qin ? __ldcg(a.qin + item) : (int32_t)item;
+    for (int64_t item = gwarp; item < count; item += nwarps) {
+        const int32_t qi = a.qin ? a.qin[item] : (int32_t)item;
         const int32_t p = a.queries ? a.queries[qi] : qi;
-        float R = a.qin ? __ldcg(a.radius + qi) : a.seed_h[qi] * a.radius_factor;
+        float R = a.qin ? a.radius[qi] : a.seed_h[qi] * a.radius_factor;
         // a negative queued radius was set by the block-wide path from a histogram
         // of the distances: it holds at least k and at most a buffer, so it is
         // scanned by this warp whatever the size of its scan list
         const bool cert = a.qin && R < 0.0f;
         R = fabsf(R);
         if (!(R > 0.0f) || !isfinite(R)) R = side * 1e-3f;
-        float rlo = a.qin ? __ldcg(a.rlo + qi) : 0.0f, rhi = a.qin ? __ldcg(a.rhi + qi) : 0.0f;
+        float rlo = a.qin ? a.rlo[qi] : 0.0f, rhi = a.qin ? a.rhi[qi] : 0.0f;
         const float4 h0 = a.hi[p], l0 = a.lo[p];
 
         // ---- level and cell box ------------------------------------------
@@ -752,8 +940,6 @@ __device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *k
             }
             __syncwarp();
         }
-        KNN_TICK(t_b);
-        KNN_PHASE(0, t_a, t_b);
         // prune to the non-empty cells that meet this query's sphere
         int nlist = 0;
         KNN_LOOP_HINT
@@ -822,23 +1008,7 @@ __device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *k
             nlist = w;
             if (lane == 0) S.off[nlist] = (uint32_t)total;
             __syncwarp();
-#ifdef MG_KNN_DEBUG
-            // scan-list entries must be disjoint slot ranges
-            for (int e = lane; e < nlist; e += 32) {
-                const uint32_t ea = S.pa[e], eb = S.pa[e] + (S.off[e + 1] - S.off[e]);
-                for (int j = 0; j < nlist; ++j) {
-                    const uint32_t ja = S.pa[j], jb = S.pa[j] + (S.off[j + 1] - S.off[j]);
-                    if (j != e && ea < jb && ja < eb) {
-                        atomicAdd((unsigned long long *)&a.stats[15], 1ull);
-                        atomicMax((unsigned long long *)&a.stats[14], (unsigned long long)qi);
-                    }
-                }
-            }
-            __syncwarp();
-#endif
             st.cand += total;
-            KNN_TICK(t_c);
-            KNN_PHASE(1, t_b, t_c);
             // ---- gather candidates with d^2 <= R^2 -------------------------
             // mode 0 fills the buffer; modes 1..3 (only after an overflow) scan
             // again and histogram the in-radius candidates so the next radius
@@ -902,11 +1072,6 @@ __device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *k
                                                 k, kKnnCap);
             }
 
-            KNN_TICK(t_d);
-            KNN_PHASE(2, t_c, t_d);
-#ifdef MG_KNN_PROFILE
-            if (total > 8192) st.phase[5] += 1;  // big single-warp scans
-#endif
             // ---- radius updates (bracketed) ------------------------------------
             // rlo: largest radius seen holding fewer than k; rhi: smallest radius
             // seen holding more than the buffer (so at least k).  Growth is a
@@ -944,8 +1109,6 @@ __device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *k
                 }
             }
 
-            KNN_TICK(t_e);
-            KNN_PHASE(3, t_d, t_e);
             if (Rnew > 0.0f) {
                 st.reason[reason - 1] += 1;
                 if (a.last_pass) {
@@ -997,20 +1160,8 @@ __device__ __forceinline__ void knn_warp_pass(const KnnArgs &a, unsigned char *k
         for (int r = 0; r < 3; ++r)
             if (st.reason[r]) atomicAdd((unsigned long long *)&a.stats[6 + r], (unsigned long long)st.reason[r]);
         if (st.heavy) atomicAdd((unsigned long long *)&a.stats[9], (unsigned long long)st.heavy);
-#ifdef MG_KNN_PROFILE
-        for (int r = 0; r < 6; ++r)
-            if (r != 4 && st.phase[r]) atomicAdd((unsigned long long *)&a.stats[10 + r], (unsigned long long)st.phase[r]);
-        atomicMax((unsigned long long *)&a.stats[14], (unsigned long long)(clock64() - t_warp0));  // slowest warp
-#endif
     }
 }
-
-template <int DIM, int KPL>
-__global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_hsml(const __grid_constant__ KnnArgs a) {
-    extern __shared__ __align__(16) unsigned char knn_smem[];
-    knn_warp_pass<DIM, KPL>(a, knn_smem);
-}
-
 
 // ---- heavy queries: one block per query ------------------------------------------
 // A query whose scan list holds more than kHeavy particles (a dense clump inside
@@ -1038,12 +1189,13 @@ struct HeavySmem {
 };
 
 template <int DIM, int KPL>
-__device__ __forceinline__ void knn_heavy_pass(const KnnArgs &a, HeavySmem<KPL> &H) {
+__global__ __launch_bounds__(kHeavyThreads) void k_knn_heavy(const __grid_constant__ KnnPassArgs a) {
+    __shared__ HeavySmem<KPL> H;
     constexpr int kCap = KnnSmem<KPL>::kCap;
     static_assert(kHeavyBins == 4 * kHeavyThreads, "four bins per thread");
     static_assert(2 * kCap <= kHeavyBins, "sort scratch lives in the histogram");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int navail = min(__ldcg(a.heavy_count), a.heavy_cap);  // written by the warp path (L2 reads, as there)
+    const int navail = min(*a.heavy_count, a.heavy_cap);
     const Frame fr = load_frame(a.frame);
     const int k = a.k;
     WarpStats st;
@@ -1053,16 +1205,16 @@ __device__ __forceinline__ void knn_heavy_pass(const KnnArgs &a, HeavySmem<KPL> 
         const int h = H.item;
         if (h >= navail) break;
         const int32_t *item = a.heavy + (int64_t)h * kHeavyItem;
-        const int32_t qi = __ldcg(item);
-        const int nlist = __ldcg(item + 1);
-        for (int e = tid; e < nlist; e += kHeavyThreads) H.pa[e] = (uint32_t)__ldcg(item + 2 + e);
-        for (int e = tid; e <= nlist; e += kHeavyThreads) H.off[e] = (uint32_t)__ldcg(item + 2 + kList + e);
+        const int32_t qi = item[0];
+        const int nlist = item[1];
+        for (int e = tid; e < nlist; e += kHeavyThreads) H.pa[e] = (uint32_t)item[2 + e];
+        for (int e = tid; e <= nlist; e += kHeavyThreads) H.off[e] = (uint32_t)item[2 + kList + e];
         __syncthreads();
         const int total = (int)H.off[nlist];
         const int32_t p = a.queries ? a.queries[qi] : qi;
         const float4 h0 = a.hi[p], l0 = a.lo[p];
-        const float R = __ldcg(a.radius + qi);
-        float rlo = __ldcg(a.rlo + qi), rhi = __ldcg(a.rhi + qi);
+        const float R = a.radius[qi];
+        float rlo = a.rlo[qi], rhi = a.rhi[qi];
         const float R2 = R * R, invR2 = 1.0f / R2;
         // candidate g of the flattened list -> slot (largest entry with off <= g)
         auto slot_of = [&](int g) -> uint32_t {
@@ -1184,14 +1336,6 @@ __device__ __forceinline__ void knn_heavy_pass(const KnnArgs &a, HeavySmem<KPL> 
             }
             __syncthreads();
             const int cnt = H.cnt;
-#ifdef MG_KNN_DEBUG
-            for (int e = tid; e < min(cnt, kCap); e += kHeavyThreads)
-                for (int j = 0; j < min(cnt, kCap); ++j)
-                    if (j != e && H.S.i[j] == H.S.i[e]) {
-                        atomicAdd((unsigned long long *)&a.stats[13], 1ull);
-                        atomicMax((unsigned long long *)&a.stats[12], (unsigned long long)qi);
-                    }
-#endif
             if (cnt < k || cnt > kCap) {
                 // rounding at the bin edge or ties finer than the bins: the warp
                 // path scans this radius and handles the overflow itself
@@ -1255,55 +1399,342 @@ __device__ __forceinline__ void knn_heavy_pass(const KnnArgs &a, HeavySmem<KPL> 
     }
 }
 
-template <int DIM, int KPL>
-__global__ __launch_bounds__(kHeavyThreads) void k_knn_heavy(const __grid_constant__ KnnArgs a) {
-    __shared__ HeavySmem<KPL> H;
-    knn_heavy_pass<DIM, KPL>(a, H);
-}
-
-// ---- the warp passes as one cooperative launch --------------------------------
-// Passes 1 .. npass - 1 of the host loop below in one kernel: each pass runs
-// the warp path over the queue the previous pass left, a grid-wide barrier,
-// the block-wide path over the heavy queries the warps handed over, and a
-// second barrier; the loop ends when a pass starts on an empty queue (every
-// block reads the same count after the barrier, so all leave together).  The
-// pass's queue pointers are set in a shared copy of the arguments.  Shared
-// memory holds the warps' buffers and, in turn, the block-wide path's.
-struct PassQueues {
-    int32_t *qa, *qb, *counts, *hcounts, *hnext;
-    int npass, max_passes;
-};
-
-__device__ __forceinline__ void set_pass(KnnArgs &sa, const PassQueues &pq, int pass) {
-    sa.qin = pass % 2 ? pq.qa : pq.qb;
-    sa.qin_count = pq.counts + (pass - 1);
-    sa.qout = pass % 2 ? pq.qb : pq.qa;
-    sa.qout_count = pq.counts + pass;
-    sa.last_pass = pass == pq.max_passes - 1;
-    sa.heavy_count = pq.hcounts + pass;
-    sa.heavy_next = pq.hnext + pass;
-}
-
-template <int DIM, int KPL>
-__global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_passes(const __grid_constant__ KnnArgs a,
-                                                                             const PassQueues pq) {
-    static_assert(kKnnWarps * 32 == kHeavyThreads, "one block shape for both paths");
+// Warp-per-query path: persistent warps take queries from a common counter and
+// search each until it is decided, growing or cutting its radius in place; a
+// query is not queued again for another pass.  Passing the undecided queries
+// through a queue took a launch pair and an empty-queue check per possible
+// pass (45 launches, most on an empty queue: ~0.1 ms of the 1.3 ms of a small
+// set).
+template <int DIM>
+__global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_hsml(const __grid_constant__ KnnArgs a) {
+    using SM = KnnSmem<1>;
+    constexpr int kKnnCap = SM::kCap;
     extern __shared__ __align__(16) unsigned char knn_smem[];
-    __shared__ KnnArgs sa;
-    cg::grid_group grid = cg::this_grid();
-    for (int pass = 1; pass < pq.npass; ++pass) {
-        __syncthreads();  // the previous pass is done with sa
-        if (threadIdx.x == 0) {
-            sa = a;
-            set_pass(sa, pq, pass);
+    SM &S = reinterpret_cast<SM *>(knn_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned count = a.qin ? (unsigned)*a.qin_count : (unsigned)a.nq;
+    const unsigned run = a.qin ? 1u : kRun;
+    const Frame fr = load_frame(a.frame);
+    const float side = (float)fr.side;
+    const float half_side = 0.5f * side;
+    const int k = a.k;
+
+    WarpStats st;
+#ifdef MG_KNN_PROFILE
+    const long long t_warp0 = clock64();
+#endif
+    // the cell-box ranges of the warp's previous search, reused when the next
+    // one needs the same box (consecutive queries are neighbours in Morton order)
+    int cL = -1, cmin_c[3] = {0, 0, 0}, cnum_c[3] = {0, 0, 0};  // cached box
+    for (;;) {
+    unsigned c0 = 0;
+    if (lane == 0) c0 = atomicAdd(a.next, run);
+    c0 = __shfl_sync(0xffffffffu, c0, 0);
+    if (c0 >= count) break;
+    const unsigned c1 = min(count, c0 + run);
+    for (unsigned item = c0; item < c1; ++item) {
+        const int32_t qi = a.qin ? a.qin[item] : (int32_t)item;
+        const int32_t p = a.queries ? a.queries[qi] : qi;
+        float R = a.qin ? a.radius[qi] : a.seed_h[qi] * a.radius_factor;
+        if (!(R > 0.0f) || !isfinite(R)) R = side * 1e-3f;
+        // rlo: largest radius seen holding fewer than k; rhi: smallest radius
+        // seen holding more than the buffer (so at least k); 0: none
+        float rlo = 0.0f, rhi = 0.0f;
+        const float4 h0 = a.hi[p], l0 = a.lo[p];
+        bool listed = false;  // the scan list is complete for this radius
+        int nlist = 0, total = 0;
+        for (int tries = 1;; ++tries) {
+        KNN_TICK(t_a);
+        if (!listed) {
+        // ---- level and cell box ------------------------------------------
+        // level_bias 1 allows R up to two cell sides, so with the rounding
+        // margin of rc a box can reach 6 cells per axis; a box over kList
+        // cells (the per-warp cache) is redone one level coarser (<= 4 per axis)
+        int L = (int)floorf(log2f(side / R)) + a.level_bias;
+        L = max(0, min(kMaxLevel, L));
+        float cells_per_side, scale, u[3], rc;
+        int cmin[3], cnum[3], ncell;
+        bool full[3];  // periodic axis covered entirely: no distance test
+        for (;;) {
+            cells_per_side = (float)(1u << L);
+            scale = cells_per_side / side;
+            u[0] = ((h0.x + half_side) + l0.x) * scale;
+            u[1] = ((h0.y + half_side) + l0.y) * scale;
+            u[2] = ((h0.z + half_side) + l0.z) * scale;
+            rc = R * scale * (1.0f + 1e-5f) + 1e-3f + cells_per_side * 2.4e-7f;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                full[d] = false;
+                if (d >= DIM) {
+                    cmin[d] = 0;
+                    cnum[d] = 1;
+                    continue;
+                }
+                int lo_c = (int)floorf(u[d] - rc), hi_c = (int)floorf(u[d] + rc);
+                if (a.periodic) {
+                    if (hi_c - lo_c + 1 >= (int)cells_per_side) {
+                        lo_c = 0;
+                        hi_c = (int)cells_per_side - 1;
+                        full[d] = true;
+                    }
+                } else {
+                    lo_c = max(lo_c, 0);
+                    hi_c = min(hi_c, (int)cells_per_side - 1);
+                }
+                cmin[d] = lo_c;
+                cnum[d] = max(0, hi_c - lo_c + 1);
+            }
+            ncell = cnum[0] * cnum[1] * cnum[2];
+            if (ncell <= kList || L == 0) break;
+            --L;
         }
-        __syncthreads();
-        if (__ldcg(sa.qin_count) == 0) break;  // the same value in every block (read at L2)
-        if (blockIdx.x == 0 && threadIdx.x == 0 && sa.stats) atomicAdd((unsigned long long *)&sa.stats[0], 1ull);
-        knn_warp_pass<DIM, KPL>(sa, knn_smem);
-        grid.sync();
-        knn_heavy_pass<DIM, KPL>(sa, *reinterpret_cast<HeavySmem<KPL> *>(knn_smem));
-        grid.sync();
+        const float inv_nx = 1.0f / (float)max(cnum[0], 1), inv_nxy = 1.0f / (float)max(cnum[0] * cnum[1], 1);
+
+        // ---- cell ranges: look up the box unless it is the cached one --------
+        const bool same_box = (L == cL) && cmin[0] == cmin_c[0] && cmin[1] == cmin_c[1] && cmin[2] == cmin_c[2] &&
+                              cnum[0] == cnum_c[0] && cnum[1] == cnum_c[1] && cnum[2] == cnum_c[2];
+        if (!same_box) {
+            // Cells that the previous box (same level) also held are copied from
+            // the cache instead of looked up again (consecutive queries' boxes
+            // are mostly shifted copies of each other); the new ranges are staged
+            // in the scan-list arrays, free at this point, then moved.
+            const bool shift_ok = L == cL;
+            KNN_LOOP_HINT
+            for (int cb = 0; cb < ncell; cb += 32) {
+                const int c = cb + lane;
+                if (c < ncell) {
+                    int ix, iy, iz;
+                    box_index(c, inv_nx, inv_nxy, cnum, ix, iy, iz);
+                    int gx = cmin[0] + ix, gy = cmin[1] + iy, gz = cmin[2] + iz;
+                    const int ox = gx - cmin_c[0], oy = gy - cmin_c[1], oz = gz - cmin_c[2];
+                    uint32_t ca, cbnd;
+                    if (shift_ok && ox >= 0 && ox < cnum_c[0] && oy >= 0 && oy < cnum_c[1] && oz >= 0 &&
+                        oz < cnum_c[2]) {
+                        const int oc = ox + cnum_c[0] * (oy + cnum_c[1] * oz);
+                        ca = S.ca[oc];
+                        cbnd = S.cb[oc];
+                    } else {
+                        const int M = (int)cells_per_side;
+                        if (a.periodic) {
+                            gx = ((gx % M) + M) % M;
+                            gy = ((gy % M) + M) % M;
+                            gz = ((gz % M) + M) % M;
+                        }
+                        if (DIM < 3) gz = 0;
+                        if (DIM < 2) gy = 0;
+                        cell_range(a.ci, L, (uint32_t)gx, (uint32_t)gy, (uint32_t)gz, ca, cbnd);
+                    }
+                    S.pa[c] = ca;
+                    S.pb[c] = cbnd;
+                }
+            }
+            __syncwarp();
+            KNN_LOOP_HINT
+            for (int c = lane; c < ncell; c += 32) {
+                S.ca[c] = S.pa[c];
+                S.cb[c] = S.pb[c];
+            }
+            cL = L;
+            for (int d = 0; d < 3; ++d) {
+                cmin_c[d] = cmin[d];
+                cnum_c[d] = cnum[d];
+            }
+            __syncwarp();
+        }
+        KNN_TICK(t_b);
+        KNN_PHASE(0, t_a, t_b);
+        // prune to the non-empty cells that meet this query's sphere
+        nlist = 0;
+        int listed_total = 0;
+        const uint32_t gofs = a.periodic ? (uint32_t)cells_per_side : 0u;
+        KNN_LOOP_HINT
+        for (int cb = 0; cb < ncell; cb += 32) {
+            const int c = cb + lane;
+            bool use = false;
+            uint32_t ca = 0, cbnd = 0;
+            int gx = 0, gy = 0, gz = 0;
+            if (c < ncell) {
+                ca = S.ca[c];
+                cbnd = S.cb[c];
+                int ix, iy, iz;
+                box_index(c, inv_nx, inv_nxy, cnum, ix, iy, iz);
+                gx = cmin[0] + ix;
+                gy = cmin[1] + iy;
+                gz = cmin[2] + iz;
+                float dx = full[0] ? 0.0f : fmaxf(0.0f, fmaxf((float)gx - u[0], u[0] - (float)(gx + 1)));
+                float dy = full[1] ? 0.0f : fmaxf(0.0f, fmaxf((float)gy - u[1], u[1] - (float)(gy + 1)));
+                float dz = full[2] ? 0.0f : fmaxf(0.0f, fmaxf((float)gz - u[2], u[2] - (float)(gz + 1)));
+                if (DIM < 3) dz = 0.0f;
+                if (DIM < 2) dy = 0.0f;
+                use = cbnd > ca && dx * dx + dy * dy + dz * dz <= rc * rc;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, use);
+            const int pos = nlist + __popc(m & ((1u << lane) - 1u));
+            if (use) {
+                S.pa[pos] = ca;
+                S.pb[pos] = cbnd;
+                S.pc[pos] = (uint64_t)L | ((uint64_t)((uint32_t)gx + gofs) << 5) |
+                            ((uint64_t)((uint32_t)gy + gofs) << 24) | ((uint64_t)((uint32_t)gz + gofs) << 43);
+            }
+            nlist += __popc(m);
+            listed_total += __reduce_add_sync(0xffffffffu, use ? (int)(cbnd - ca) : 0);
+        }
+        __syncwarp();
+        // (a coordinate of the list holds 19 bits: three boxes of level 17)
+        if (listed_total > kNarrow && (!a.periodic || L < kMaxLevel)) {
+            float Rl = R * scale;
+            const float R0 = Rl;
+            const int fm = (full[0] ? 1 : 0) | (full[1] ? 2 : 0) | (full[2] ? 4 : 0);
+            nlist = narrow_list<DIM>(S, a, p, nlist, kNarrow / 2, L, u[0], u[1], u[2], fm, scale,
+                                     1e-3f + cells_per_side * 2.4e-7f, Rl);
+            if (Rl < R0) R = Rl / scale;
+            st.heavy += 1;
+        }
+        // drop emptied entries and form prefix offsets (entries strictly non-empty)
+        {
+            int w = 0;
+            total = 0;
+            KNN_LOOP_HINT
+            for (int i0 = 0; i0 < nlist; i0 += 32) {
+                const int i = i0 + lane;
+                const uint32_t ra = i < nlist ? S.pa[i] : 0u, rb = i < nlist ? S.pb[i] : 0u;
+                const int n_i = (int)(rb - ra);
+                __syncwarp();
+                const unsigned m = __ballot_sync(0xffffffffu, n_i > 0);
+                const int inc = warp_incl_scan(n_i);
+                if (n_i > 0) {
+                    const int pos = w + __popc(m & ((1u << lane) - 1u));
+                    S.pa[pos] = ra;
+                    S.pb[pos] = rb;
+                    S.off[pos] = (uint32_t)(total + inc - n_i);
+                }
+                w += __popc(m);
+                total += __shfl_sync(0xffffffffu, inc, 31);
+            }
+            nlist = w;
+            if (lane == 0) S.off[nlist] = (uint32_t)total;
+            __syncwarp();
+        }
+        st.cand += total;
+        listed = true;
+        }
+        KNN_TICK(t_c);
+        KNN_PHASE(1, t_a, t_c);
+        // ---- gather candidates with d^2 <= R^2 -------------------------
+        // More than the buffer holds: the rest is binned, and the radius is cut
+        // to the bucket that holds the k-th neighbour.  More than kScanLimit
+        // particles in the list (before any radius of this query has held
+        // fewer than k): no scan, the radius shrinks by the volume ratio.
+        int cnt = 0;
+        const float R2 = R * R, invR2 = 1.0f / R2;
+        const bool too_big = total > kScanLimit && rlo == 0.0f;
+        float v_hi = 1.0f;
+        if (!too_big) {
+            int j0 = 0;
+            KNN_LOOP_HINT
+            for (int g0 = 0; g0 < total; g0 += 32) {
+                const uint32_t t = chunk_slot(S, nlist, total, g0, j0, lane);
+                const float dd = g0 + lane < total ? cand_d2(a, h0, l0, t) : FLT_MAX;
+                const bool in = dd <= R2;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                const int pos = cnt + __popc(m & ((1u << lane) - 1u));
+                if (in && pos < kKnnCap) {
+                    S.d[pos] = dd;
+                    S.i[pos] = (int32_t)t;
+                }
+                const int before = cnt;
+                cnt += __popc(m);
+                // Lazy histogram: the first time the buffer overflows, the
+                // buffered candidates are binned; from then on every new
+                // in-radius candidate is binned directly, so an overflow
+                // usually needs no second scan.
+                if (before <= kKnnCap && cnt > kKnnCap) lazy_hist_init<DIM>(S, invR2);
+                if (cnt > kKnnCap && in && pos >= kKnnCap) atomicAdd(&S.hist[(int)bucket_of(dd * invR2, DIM)], 1);
+            }
+            __syncwarp();
+            if (cnt > kKnnCap)
+                v_hi = overflow_window<DIM>(S, a.hi, a.lo, a.periodic, a.box_hi, a.box_lo, h0, l0, nlist, total, R2,
+                                            k, kKnnCap);
+        }
+        KNN_TICK(t_d);
+        KNN_PHASE(2, t_c, t_d);
+        // ---- radius updates (bracketed) ------------------------------------
+        // Growth is a geometric guess capped by rhi (geometric mean once both
+        // are known); an overflow cuts the radius to the histogram bucket
+        // holding the k-th neighbour, which holds at least k by construction,
+        // and scans the same list again.
+        float Rnew = -1.0f;
+        int reason = 0;
+        if (too_big) {
+            Rnew = R * fmaxf(0.25f, powf(0.5f * kKnnCap / (float)total, 1.0f / DIM));
+            reason = 2;
+            listed = false;
+        } else if (cnt < k) {
+            rlo = fmaxf(rlo, R);
+            const float g = 1.25f * powf((float)k / (float)max(cnt, 1), 1.0f / DIM);
+            Rnew = R * fminf(fmaxf(g, 1.25f), 4.0f);
+            if (rhi > 0.0f && Rnew >= rhi) Rnew = sqrtf(rlo * rhi);
+            reason = 1;
+            listed = false;
+        } else if (cnt > kKnnCap) {
+            rhi = (rhi > 0.0f) ? fminf(rhi, R) : R;
+            Rnew = R * (DIM == 3 ? cbrtf(v_hi) : (DIM == 2 ? sqrtf(v_hi) : v_hi)) * 1.00001f;
+            if (Rnew >= R) Rnew = R * 0.999f;
+            reason = 2;
+        }
+        // ---- select the k smallest: bucket histogram ------------------------
+        float T = 0.0f;
+        if (Rnew < 0.0f) {
+            T = select_k<DIM>(S, cnt, invR2, k, a.ngb + (int64_t)qi * k);
+            // the band around T must lie inside the searched radius
+            const float wabs = band_abs(T, query_mag(a.hi, p, a.periodic, a.box_hi));
+            if (T * (1.0f + kBandEps) + 2.0f * wabs > R2) {
+                Rnew = sqrtf(T * (1.0f + 2.0f * kBandEps) + 4.0f * wabs) * 1.0001f;
+                reason = 3;
+                listed = false;  // (the selection used the list's memory)
+            }
+        }
+        KNN_TICK(t_e);
+        KNN_PHASE(3, t_d, t_e);
+        if (!(Rnew > 0.0f)) {
+            finish_row(S, cnt, T, k, p, qi, a, fr.side, st);
+            st.tries = max(st.tries, tries - 1);
+            break;
+        }
+        st.reason[reason - 1] += 1;
+        if (tries >= a.max_tries) {
+            if (lane == 0) {
+                atomicOr(a.qstatus + qi, MG_Q_UNRESOLVED);
+                // diagnostics for the caller: last radius and candidate count
+                a.radius[qi] = R;
+                a.hsml[qi] = -(float)((too_big ? total : cnt) + 1000000 * reason);
+            }
+            st.unres += 1;
+            break;
+        }
+        st.retry += 1;
+        R = Rnew;
+        __syncwarp();
+        }
+    }
+    }
+
+    // statistics: one atomic per warp
+    if (lane == 0 && a.stats) {
+        if (st.tries) atomicMax((unsigned long long *)&a.stats[0], (unsigned long long)st.tries);
+        if (st.cand) atomicAdd((unsigned long long *)&a.stats[1], (unsigned long long)st.cand);
+        if (st.retry) atomicAdd((unsigned long long *)&a.stats[2], (unsigned long long)st.retry);
+        if (st.band) atomicAdd((unsigned long long *)&a.stats[3], (unsigned long long)st.band);
+        if (st.unres) atomicAdd((unsigned long long *)&a.stats[4], (unsigned long long)st.unres);
+        if (st.newton) atomicAdd((unsigned long long *)&a.stats[5], (unsigned long long)st.newton);
+        for (int r = 0; r < 3; ++r)
+            if (st.reason[r]) atomicAdd((unsigned long long *)&a.stats[6 + r], (unsigned long long)st.reason[r]);
+        if (st.heavy) atomicAdd((unsigned long long *)&a.stats[9], (unsigned long long)st.heavy);
+#ifdef MG_KNN_PROFILE
+        for (int r = 0; r < 6; ++r)
+            if (r != 4 && st.phase[r]) atomicAdd((unsigned long long *)&a.stats[10 + r], (unsigned long long)st.phase[r]);
+        atomicMax((unsigned long long *)&a.stats[14], (unsigned long long)(clock64() - t_warp0));  // slowest warp
+#endif
     }
 }
 
@@ -2008,8 +2439,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             Rnew = fmaxf(R, sqrtf(T) + 4.0f * (1.01f * eg + 2e-7f * R)) * 1.0001f;
         }
         a.radius[qi] = Rnew;
-        a.rlo[qi] = 0.0f;
-        a.rhi[qi] = 0.0f;
     }
     const unsigned pm = __ballot_sync(0xffffffffu, push);
     if (pm) {
@@ -2562,37 +2991,30 @@ __global__ __launch_bounds__(256) void k_neighbor_dist(const double *__restrict_
 
 using namespace mg;
 
-template <int DIM, int KPL>
-static int launch_knn_t(unsigned blocks, size_t, cudaStream_t st, const KnnArgs &a) {
-    const size_t smem = sizeof(KnnSmem<KPL>) * kKnnWarps;
-    MG_CUDA(cudaFuncSetAttribute(k_knn_hsml<DIM, KPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_knn_hsml<DIM, KPL><<<blocks, kKnnWarps * 32, smem, st>>>(a);
-    return MG_OK;
-}
-
 template <int DIM>
-static int launch_knn_d(int kpl, unsigned blocks, size_t smem, cudaStream_t st, const KnnArgs &a) {
-    if (kpl == 1) return launch_knn_t<DIM, 1>(blocks, smem, st, a);
-    if (kpl == 2) return launch_knn_t<DIM, 2>(blocks, smem, st, a);
-    return launch_knn_t<DIM, 4>(blocks, smem, st, a);
-}
-
-template <int DIM>
-static int launch_heavy_d(int kpl, unsigned blocks, cudaStream_t st, const KnnArgs &a) {
-    if (kpl == 1)
-        k_knn_heavy<DIM, 1><<<blocks, kHeavyThreads, 0, st>>>(a);
-    else if (kpl == 2)
-        k_knn_heavy<DIM, 2><<<blocks, kHeavyThreads, 0, st>>>(a);
-    else
-        k_knn_heavy<DIM, 4><<<blocks, kHeavyThreads, 0, st>>>(a);
+static int launch_knn_d(unsigned blocks, cudaStream_t st, const KnnArgs &a) {
+    const size_t smem = sizeof(KnnSmem<1>) * kKnnWarps;
+    MG_CUDA(cudaFuncSetAttribute(k_knn_hsml<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_knn_hsml<DIM><<<blocks, kKnnWarps * 32, smem, st>>>(a);
     MG_CHECK_LAUNCH();
     return MG_OK;
 }
 
-static int launch_heavy(int dim, int kpl, unsigned blocks, cudaStream_t st, const KnnArgs &a) {
-    if (dim == 1) return launch_heavy_d<1>(kpl, blocks, st, a);
-    if (dim == 2) return launch_heavy_d<2>(kpl, blocks, st, a);
-    return launch_heavy_d<3>(kpl, blocks, st, a);
+template <int DIM, int KPL>
+static int launch_pass_t(unsigned blocks, unsigned heavy_blocks, cudaStream_t st, const KnnPassArgs &a) {
+    const size_t smem = sizeof(KnnSmem<KPL>) * kKnnWarps;
+    MG_CUDA(cudaFuncSetAttribute(k_knn_pass<DIM, KPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_knn_pass<DIM, KPL><<<blocks, kKnnWarps * 32, smem, st>>>(a);
+    MG_CHECK_LAUNCH();
+    k_knn_heavy<DIM, KPL><<<heavy_blocks, kHeavyThreads, 0, st>>>(a);
+    MG_CHECK_LAUNCH();
+    return MG_OK;
+}
+
+template <int DIM>
+static int launch_pass_d(int k, unsigned blocks, unsigned heavy_blocks, cudaStream_t st, const KnnPassArgs &a) {
+    return k <= 64 ? launch_pass_t<DIM, 2>(blocks, heavy_blocks, st, a)
+                   : launch_pass_t<DIM, 4>(blocks, heavy_blocks, st, a);
 }
 
 #ifndef MG_KNN_GROUP_G
@@ -2628,65 +3050,23 @@ extern "C" int mg_knn_set_group_pass(int32_t enabled) {
     return g_group_pass.exchange(enabled ? 1 : 0);
 }
 
-// process-wide switch of the cooperative launch of the warp passes; off (the
-// default): the host loop of one launch per kernel and pass.  Measured on a
-// GB300, the cooperative launch gives the same answers; the search + h stage
-// of 2^22 Plummer takes the same time either way (10.72-10.85 against
-// 10.78-10.83 ms over two runs), of the 2^24 clump mixture longer (74.6-75.7
-// against 72.1-73.4 ms: one wave of resident blocks balances the queue worse
-// than two), and a grid that holds every SM keeps the snapshot lanes of a
-// batch from overlapping (64 snapshots: 271 against 207 ms).
+// The warp path is launched the same way whatever this is set to.  It keeps its setting for its callers.
 static std::atomic<int> g_persistent_passes{0};
 
 extern "C" int mg_knn_set_persistent_passes(int32_t enabled) {
     return g_persistent_passes.exchange(enabled ? 1 : 0);
 }
 
-// Passes 1 .. pq.npass - 1 in one cooperative launch (k_knn_passes), one wave
-// of the blocks the SMs hold at once; done = false when the device cannot
-// take it (no cooperative launch, no resident block), and the caller runs the
-// host loop instead.
-template <int DIM, int KPL>
-static int launch_passes_t(int nsm, cudaStream_t st, const KnnArgs &a, const PassQueues &pq, bool &done) {
-    done = false;
-    const size_t smem = std::max(sizeof(KnnSmem<KPL>) * kKnnWarps, sizeof(HeavySmem<KPL>));
-    auto fn = k_knn_passes<DIM, KPL>;
-    MG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kKnnWarps * 32, smem));
-    if (per_sm < 1) return MG_OK;
-    KnnArgs aa = a;
-    PassQueues qq = pq;
-    void *args[] = {&aa, &qq};
-    MG_CUDA(cudaLaunchCooperativeKernel((const void *)fn, dim3((unsigned)(nsm * per_sm)), dim3(kKnnWarps * 32), args,
-                                        smem, st));
-    done = true;
-    return MG_OK;
+static int launch_knn(int dim, unsigned blocks, cudaStream_t st, const KnnArgs &a) {
+    if (dim == 1) return launch_knn_d<1>(blocks, st, a);
+    if (dim == 2) return launch_knn_d<2>(blocks, st, a);
+    return launch_knn_d<3>(blocks, st, a);
 }
 
-template <int DIM>
-static int launch_passes_d(int kpl, int nsm, cudaStream_t st, const KnnArgs &a, const PassQueues &pq, bool &done) {
-    if (kpl == 1) return launch_passes_t<DIM, 1>(nsm, st, a, pq, done);
-    if (kpl == 2) return launch_passes_t<DIM, 2>(nsm, st, a, pq, done);
-    return launch_passes_t<DIM, 4>(nsm, st, a, pq, done);
-}
-
-static int launch_passes(int dim, int kpl, int nsm, cudaStream_t st, const KnnArgs &a, const PassQueues &pq,
-                         bool &done) {
-    done = false;
-    int dev = 0, coop = 0;
-    MG_CUDA(cudaGetDevice(&dev));
-    MG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop || !g_persistent_passes.load()) return MG_OK;
-    if (dim == 1) return launch_passes_d<1>(kpl, nsm, st, a, pq, done);
-    if (dim == 2) return launch_passes_d<2>(kpl, nsm, st, a, pq, done);
-    return launch_passes_d<3>(kpl, nsm, st, a, pq, done);
-}
-
-static int launch_knn(int dim, int kpl, unsigned blocks, size_t smem, cudaStream_t st, const KnnArgs &a) {
-    if (dim == 1) return launch_knn_d<1>(kpl, blocks, smem, st, a);
-    if (dim == 2) return launch_knn_d<2>(kpl, blocks, smem, st, a);
-    return launch_knn_d<3>(kpl, blocks, smem, st, a);
+static int launch_pass(int dim, unsigned blocks, unsigned heavy_blocks, cudaStream_t st, const KnnPassArgs &a) {
+    if (dim == 1) return launch_pass_d<1>(a.k, blocks, heavy_blocks, st, a);
+    if (dim == 2) return launch_pass_d<2>(a.k, blocks, heavy_blocks, st, a);
+    return launch_pass_d<3>(a.k, blocks, heavy_blocks, st, a);
 }
 
 static inline CellIndex make_index(const mg_cells *c) {
@@ -2724,10 +3104,49 @@ extern "C" size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k) {
     if (nq <= 0 || k < 1) return 0;
     // the selected-distance rows are scratch of the h solve only for k > 32
     const size_t dsel_entries = k > 32 ? (size_t)nq * (size_t)k : 0;
-    return 3 * align_up(sizeof(float) * nq) + 2 * align_up(sizeof(int32_t) * nq) +
-           align_up(sizeof(float) * dsel_entries) +
-           align_up(sizeof(int32_t) * (size_t)heavy_capacity(nq) * kHeavyItem) + 3 * align_up(sizeof(int32_t) * 64) +
-           1024;
+    size_t b = align_up(sizeof(float) * nq) + align_up(sizeof(int32_t) * nq) + align_up(sizeof(int32_t) * 64) + 1024;
+    if (k > 32)  // brackets, second queue, heavy items and their counters
+        b += align_up(sizeof(float) * dsel_entries) + 2 * align_up(sizeof(float) * nq) +
+             align_up(sizeof(int32_t) * nq) + align_up(sizeof(int32_t) * (size_t)heavy_capacity(nq) * kHeavyItem) +
+             2 * align_up(sizeof(int32_t) * 64);
+    return b;
+}
+
+// The search of k > 32: max_passes passes over the queue.
+static int knn_passes(const mg_cells *c, const KnnArgs &a0, int max_passes, int nsm, int32_t *counts, Carve &w,
+                      cudaStream_t st) {
+    KnnPassArgs a;
+    static_cast<KnnArgs &>(a) = a0;
+    const int64_t nq = a.nq, hcap = heavy_capacity(nq);
+    int32_t *qa = a.qout;
+    a.rlo = w.take<float>(nq);
+    a.rhi = w.take<float>(nq);
+    int32_t *qb = w.take<int32_t>(nq);
+    a.heavy = w.take<int32_t>((size_t)hcap * kHeavyItem);
+    a.heavy_cap = (int)hcap;
+    int32_t *hcounts = w.take<int32_t>(64), *hnext = w.take<int32_t>(64);
+    if (!w.ok()) return MG_ERR_ARG;
+    MG_CUDA(cudaMemsetAsync(hcounts, 0, sizeof(int32_t) * 64, st));
+    MG_CUDA(cudaMemsetAsync(hnext, 0, sizeof(int32_t) * 64, st));
+    const int npass = std::min(max_passes, 63);
+    for (int pass = 0; pass < npass; ++pass) {
+        a.qin = pass == 0 ? nullptr : (pass % 2 ? qa : qb);
+        a.qin_count = pass == 0 ? nullptr : counts + (pass - 1);
+        a.qout = pass % 2 ? qb : qa;
+        a.qout_count = counts + pass;
+        a.last_pass = pass == max_passes - 1;
+        a.heavy_count = hcounts + pass;
+        a.heavy_next = hnext + pass;
+        // the first pass over all queries, the others persistent over the queue
+        const int64_t blocks = pass == 0 ? (nq + kKnnWarps * kChunk - 1) / (kKnnWarps * kChunk) : (int64_t)nsm * 8;
+        if (pass > 0) {
+            k_count_pass<<<1, 32, 0, st>>>(counts + (pass - 1), a.stats);
+            MG_CHECK_LAUNCH();
+        }
+        const int rc = launch_pass(c->dim, (unsigned)std::min<int64_t>(blocks, 2147483647), (unsigned)nsm * 4, st, a);
+        if (rc) return rc;
+    }
+    return MG_OK;
 }
 
 extern "C" int mg_knn_hsml(const mg_cells *c, const int32_t *queries, int64_t nq, int32_t k,
@@ -2742,21 +3161,12 @@ extern "C" int mg_knn_hsml(const mg_cells *c, const int32_t *queries, int64_t nq
     if (workspace_bytes < mg_knn_hsml_workspace_bytes(nq, k)) return MG_ERR_ARG;
     cudaStream_t st = as_stream(stream_);
     Carve w(workspace, workspace_bytes);
-    float *radius = w.take<float>(nq);
-    float *rlo = w.take<float>(nq);
-    float *rhi = w.take<float>(nq);
-    int32_t *qa = w.take<int32_t>(nq);
-    int32_t *qb = w.take<int32_t>(nq);
-    int32_t *counts = w.take<int32_t>(64);
+    float *radius = w.take<float>(nq);  // first: the caller's diagnostics read it
+    int32_t *queue = w.take<int32_t>(nq);
+    int32_t *counts = w.take<int32_t>(64);  // queued queries (of each pass), next query to take
     float *dsel = w.take<float>(k > 32 ? (size_t)nq * (size_t)k : 0);
-    const int64_t hcap = heavy_capacity(nq);
-    int32_t *heavy = w.take<int32_t>((size_t)hcap * kHeavyItem);
-    int32_t *hcounts = w.take<int32_t>(64);
-    int32_t *hnext = w.take<int32_t>(64);
     if (!w.ok()) return MG_ERR_ARG;
     MG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * 64, st));
-    MG_CUDA(cudaMemsetAsync(hcounts, 0, sizeof(int32_t) * 64, st));
-    MG_CUDA(cudaMemsetAsync(hnext, 0, sizeof(int32_t) * 64, st));
     MG_CUDA(cudaMemsetAsync(qstatus, 0, sizeof(int32_t) * nq, st));
     KnnArgs a;
     fill_args(a, c);
@@ -2767,58 +3177,38 @@ extern "C" int mg_knn_hsml(const mg_cells *c, const int32_t *queries, int64_t nq
     a.radius_factor = radius_factor;
     a.level_bias = level_bias < 0 ? 0 : (level_bias > 1 ? 1 : level_bias);  // <= 5 cells per axis
     a.radius = radius;
-    a.rlo = rlo;
-    a.rhi = rhi;
     a.ngb = ngb;
     a.hsml = hsml;
     a.qstatus = qstatus;
     a.stats = stats;
-    a.heavy = heavy;
-    a.heavy_cap = (int)hcap;
+    a.qin = nullptr;
+    a.qin_count = nullptr;
+    a.next = reinterpret_cast<unsigned *>(counts + 1);
+    a.qout = queue;
+    a.qout_count = counts;
+    // a pass searched every undecided query once; a few more radii are tried in
+    // place (a list is scanned again without being rebuilt), one when the
+    // caller asks for one pass
+    a.max_tries = max_passes == 1 ? 1 : 4 * std::min(max_passes, 64);
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // first pass one thread per query over block-shared candidates (not for
-    // periodic boxes or k > 32; its leftovers need a second pass)
+    // periodic boxes or k > 32; its leftovers go to the warp path)
     const bool group_first = g_group_pass.load() && !a.periodic && k <= 32 && max_passes >= 2;
-    const int kpl = k <= 32 ? 1 : (k <= 64 ? 2 : 4);
-    const int npass = std::min(max_passes, 63);
-    for (int pass = 0; pass < npass; ++pass) {
-        if (pass == 1) {
-            // the remaining passes in one cooperative launch where possible
-            PassQueues pq{qa, qb, counts, hcounts, hnext, npass, max_passes};
-            bool done = false;
-            const int rc = launch_passes(c->dim, kpl, nsm, st, a, pq, done);
-            if (rc) return rc;
-            if (done) {
-                MG_CHECK_LAUNCH();
-                break;
-            }
-        }
-        a.qin = pass == 0 ? nullptr : (pass % 2 ? qa : qb);
-        a.qin_count = pass == 0 ? nullptr : counts + (pass - 1);
-        a.qout = pass % 2 ? qb : qa;
-        a.qout_count = counts + pass;
-        a.last_pass = pass == max_passes - 1;
-        a.heavy_count = hcounts + pass;
-        a.heavy_next = hnext + pass;
-        int64_t blocks;
-        if (pass == 0)
-            blocks = (nq + kKnnWarps * kChunk - 1) / (kKnnWarps * kChunk);
-        else
-            blocks = (int64_t)nsm * 8;  // persistent sweep over the queue
-        if (blocks > 2147483647) blocks = 2147483647;
-        if (pass > 0) k_count_pass<<<1, 32, 0, st>>>(counts + (pass - 1), stats);
-        if (pass == 0 && group_first) {
-            const int rc = launch_group(c->dim, (unsigned)((nq + kGroupThreads - 1) / kGroupThreads), st, a);
-            if (rc) return rc;
-            continue;
-        }
-        const size_t smem = 0;
-        int rc = launch_knn(c->dim, kpl, (unsigned)blocks, smem, st, a);
+    if (group_first) {
+        const int rc = launch_group(c->dim, (unsigned)((nq + kGroupThreads - 1) / kGroupThreads), st, a);
         if (rc) return rc;
-        MG_CHECK_LAUNCH();
-        rc = launch_heavy(c->dim, kpl, (unsigned)nsm * 4, st, a);
+        a.qin = queue;
+        a.qin_count = counts;
+    }
+    if (k > 32) {
+        const int rc = knn_passes(c, a, max_passes, nsm, counts, w, st);
+        if (rc) return rc;
+    } else {
+        // persistent warps, as many blocks as the SMs hold at once
+        const int64_t blocks = std::min((int64_t)nsm * kKnnMinBlocks, (nq + kKnnWarps - 1) / kKnnWarps);
+        const int rc = launch_knn(c->dim, (unsigned)blocks, st, a);
         if (rc) return rc;
     }
     if (c->dim == 1) return launch_hsml_rows<1>(st, a, qstatus, nq, k, dsel, hsml, hsml_lo, stats);
