@@ -21,6 +21,7 @@
 
 #include "mg_chol.cuh"
 #include "mg_common.cuh"
+#include "mg_f32x2.cuh"
 #include "mg_ff.cuh"
 #include "mg_refine.cuh"
 
@@ -47,20 +48,6 @@ struct Basis {
 #define MG_GRAD_UNROLL 4
 #endif
 constexpr int kGradUnroll = MG_GRAD_UNROLL;  // neighbours in flight per thread in k_grad
-// MG_GRAD_MINB > 0: resident blocks of k_grad per SM its registers are cut
-// for (0: the compiler's choice); MG_GRAD_NF8 0 caps an order-1 launch at 4
-// components (more launches, fewer registers).
-#ifndef MG_GRAD_MINB
-#define MG_GRAD_MINB 0
-#endif
-#if MG_GRAD_MINB > 0
-#define MG_GRAD_BOUNDS __launch_bounds__(128, MG_GRAD_MINB)
-#else
-#define MG_GRAD_BOUNDS __launch_bounds__(128)
-#endif
-#ifndef MG_GRAD_NF8
-#define MG_GRAD_NF8 1
-#endif
 // FP32 rounding per term assumed by the order-1 sweep's error estimate,
 // e ~ EB cond sum_j w |f_j - f_i| / |b| relative to x.  The estimate takes every
 // rounding error aligned with the direction the matrix amplifies most; with
@@ -100,13 +87,14 @@ struct GradArgs {
     int32_t *fix_queue;
     int32_t *fix_count;
     int32_t *fix_mark;  // per query: already queued (several component chunks may flag it)
+    int vec_d1;         // order 1: results stored 16 bytes at a time
     int refine;         // order 2: refine the FP32 answer once instead of queueing it (k_grad<..., true>)
 };
 
 // cholesky, chol_solve and cond_estimate: mg_chol.cuh
 
 template <int DIM, int ORDER, int NF, bool REFINE = false>
-__global__ MG_GRAD_BOUNDS void k_grad(GradArgs g) {
+__global__ __launch_bounds__(128) void k_grad(GradArgs g) {
     static_assert(!REFINE || ORDER == 2, "the refinement step is for order 2");
     using B = Basis<DIM, ORDER>;
     constexpr int ND = B::ND, NM = B::NM;
@@ -395,6 +383,262 @@ __global__ MG_GRAD_BOUNDS void k_grad(GradArgs g) {
     }
 }
 
+// ---- order 1 ------------------------------------------------------------------------
+// Up to 8 components: one thread per query (k_grad).  More: four lanes per query
+// (k_grad1).
+//
+// Four lanes per query split its neighbours for the geometry: separation,
+// kernel weight and moment matrix, with w x, w and the neighbour's slot left in
+// shared memory.  Then, for up to 16 components at a time, each lane holds one
+// group of 4 and walks all neighbours: the four lanes read 64 contiguous bytes
+// of a neighbour's row, 8 lines per warp load where one lane per query reads 32,
+// and the geometry is not repeated for the next components.  Fewer groups than
+// lanes (the last pass) leave several lanes on one group, which then split the
+// neighbours and add their compensated sums.
+//
+// Every right-hand side is summed with Kahan compensation (see k_grad).
+//
+// Bound: L1 wavefronts of the 16-byte gathers, then instruction issue.  10^6
+// Plummer particles, k = 32: 16 components 1.19 ms with 8 per launch and thread
+// -> 0.54 ms, the geometry alone ~0.4 ms of either.  With up to 8 components the
+// gathers of positions weigh most and the two forms are equal within 5% (5
+// components 0.53 / 0.58 ms), as are packed pairs in the one-thread form and
+// four lanes that each take a quarter of the neighbours through both steps.
+// 1/h as a float-float pair: the scaling of every separation by 1/h is coherent
+// across the row, and least-squares fits can be sensitive to it (1e-7 in h
+// moved some rows' order-1 answers by 1e-5); the pair carries it to ~2^-46,
+// each scaled coordinate then rounds once on its own.
+//
+// Scaled separation x of slot s from the query and the kernel weight.
+template <int DIM>
+__device__ __forceinline__ float g1_neighbour(const GradArgs &g, const float4 &h0, const float4 &l0, ff hinv, int32_t s,
+                                              float x[3]) {
+    const float4 hb = __ldg(g.hi + s), lb = __ldg(g.lo + s);
+    const float3 d = g.periodic ? sep_hilo_periodic(h0, l0, hb, lb, g.box_hi, g.box_lo) : sep_hilo(h0, l0, hb, lb);
+    x[0] = scale_sep(d.x, hinv.hi, hinv.lo);
+    x[1] = scale_sep(d.y, hinv.hi, hinv.lo);
+    x[2] = scale_sep(d.z, hinv.hi, hinv.lo);
+    float r2 = 0.0f;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) r2 += x[a] * x[a];
+    return g.weighted ? spline_w(sqrtf(r2)) : 1.0f;
+}
+
+// Factor of the moment matrix, its condition estimate, and whether the row has
+// to be re-solved in FP64 whatever its fields: no factor, a condition above the
+// threshold, or the hi/lo positions' representation error, ~1.2e-14 |x| of each
+// separation (|x| frame-relative, or the box side), above 1e-7 / cond of h.
+template <int DIM>
+__device__ __forceinline__ bool g1_factor(const GradArgs &g, const float4 &h0, float hinv,
+                                          const float M[DIM * (DIM + 1) / 2], float L[DIM * (DIM + 1) / 2],
+                                          float &cond) {
+    constexpr int NM = DIM * (DIM + 1) / 2;
+#pragma unroll
+    for (int i = 0; i < NM; ++i) L[i] = M[i];
+    bool flag = false;
+    cond = 1.0f;
+    if (!cholesky<DIM>(L)) {
+#pragma unroll
+        for (int i = 0; i < NM; ++i) L[i] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) L[i * (i + 1) / 2 + i] = 1e30f;
+        flag = true;
+    } else {
+        cond = cond_estimate<DIM>(M, L);
+        flag = cond > g.cond_thr;
+    }
+    float xq = fmaxf(fabsf(h0.x), fmaxf(fabsf(h0.y), fabsf(h0.z)));
+    if (g.periodic) xq = fmaxf(xq, g.box_hi);
+    return flag || 1.2e-14f * xq * hinv * cond > 1e-7f;
+}
+
+// Solution of one component's right-hand side b; true when the rounding of its
+// terms (cabs = sum w |f_j - f_i|) may exceed the tolerance (see k_grad).
+template <int DIM>
+__device__ __forceinline__ bool g1_solve(const float L[DIM * (DIM + 1) / 2], const float b[DIM], float cabs,
+                                         float cond, float hinv, float out[DIM]) {
+    float nb = 0.0f;
+#pragma unroll
+    for (int m = 0; m < DIM; ++m) {
+        out[m] = b[m];
+        nb += b[m] * b[m];
+    }
+    chol_solve<DIM>(L, out);
+#pragma unroll
+    for (int m = 0; m < DIM; ++m) out[m] *= hinv;
+    const float eb = MG_GRAD_EB * cond * cabs;
+    return eb * eb > 1e-5f * 1e-5f * nb;
+}
+
+// Compensated sums (r with the negated compensation nc) of the lanes o, 2 o, ..
+// up to four: error-free, the rounding joining the compensation.
+__device__ __forceinline__ void g1_merge(float &r, float &nc, int o) {
+#pragma unroll
+    for (; o < 4; o <<= 1) {
+        const float ro = __shfl_xor_sync(0xffffffffu, r, o), no = __shfl_xor_sync(0xffffffffu, nc, o);
+        float t, e;
+        two_sum(r, ro, t, e);
+        r = t;
+        nc = (nc + no) + e;
+    }
+}
+
+constexpr int kG1Queries = 32;  // queries per block of 128
+
+// Entry of neighbour j and query ql in the arrays below: queries rotated by j,
+// so that the four neighbours a query's lanes store together (j .. j + 3) fall
+// in different banks, in 16-byte and in 4-byte entries.
+__device__ __forceinline__ int g1_at(int j, int ql) { return j * kG1Queries + (ql ^ ((j & 3) * 10)); }
+
+struct G1Smem {
+    float4 *wx;  // [neighbour][query of the block]: w x, w y, w z, w
+    int32_t *s;  // [neighbour][query]: slot
+};
+
+// Components of the groups gr .. gr + WD - 1 (4 each; a group past the last
+// repeats it and is not written).
+template <int DIM, int WD>
+__device__ __forceinline__ bool g1_fields(const GradArgs &g, const G1Smem &S, int gr, int ng, int ql, int gl,
+                                          int32_t p, int64_t orow, bool valid, const float L[DIM * (DIM + 1) / 2],
+                                          float hinv, float cond) {
+    constexpr int SUBS = 4 / WD;  // lanes that share a group, each with every SUBS-th neighbour
+    const int sub = gl / WD, grp = min(gr + gl % WD, ng - 1);
+    const bool mine = valid && gr + gl % WD < ng;
+    const int c0 = 4 * grp;
+    const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
+    const ulonglong2 f0h = __ldg(reinterpret_cast<const ulonglong2 *>(g.f_hi + (int64_t)p * g.nfp + c0));
+    const ulonglong2 f0l = g.f_lo ? __ldg(reinterpret_cast<const ulonglong2 *>(g.f_lo + (int64_t)p * g.nfp + c0)) : zero;
+    unsigned long long rhs[DIM][2], ncmp[DIM][2];  // sums and their negated compensation
+    float cabs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int m = 0; m < DIM; ++m) rhs[m][0] = rhs[m][1] = ncmp[m][0] = ncmp[m][1] = 0ull;
+#pragma unroll 4
+    for (int j = sub; j < g.k; j += SUBS) {
+        const int32_t s = S.s[g1_at(j, ql)];
+        const float4 w = S.wx[g1_at(j, ql)];
+        const ulonglong2 vh = __ldg(reinterpret_cast<const ulonglong2 *>(g.f_hi + (int64_t)s * g.nfp + c0));
+        ulonglong2 vl = zero;
+        if (g.f_lo) vl = __ldg(reinterpret_cast<const ulonglong2 *>(g.f_lo + (int64_t)s * g.nfp + c0));
+        const unsigned long long d[2] = {f2_add(f2_sub(vh.x, f0h.x), f2_sub(vl.x, f0l.x)),
+                                         f2_add(f2_sub(vh.y, f0h.y), f2_sub(vl.y, f0l.y))};
+        cabs[0] += w.w * fabsf(f2_low(d[0]));
+        cabs[1] += w.w * fabsf(f2_high(d[0]));
+        cabs[2] += w.w * fabsf(f2_low(d[1]));
+        cabs[3] += w.w * fabsf(f2_high(d[1]));
+        const float wx[3] = {w.x, w.y, w.z};
+#pragma unroll
+        for (int m = 0; m < DIM; ++m) {
+            const unsigned long long wm = f2_pack(wx[m]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const unsigned long long y = f2_fma(wm, d[u], ncmp[m][u]);
+                const unsigned long long t = f2_add(rhs[m][u], y);
+                ncmp[m][u] = f2_sub(y, f2_sub(t, rhs[m][u]));
+                rhs[m][u] = t;
+            }
+        }
+    }
+    float b[4][DIM];
+#pragma unroll
+    for (int m = 0; m < DIM; ++m)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            float r[2] = {f2_low(rhs[m][u]), f2_high(rhs[m][u])}, nc[2] = {f2_low(ncmp[m][u]), f2_high(ncmp[m][u])};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (SUBS > 1) g1_merge(r[e], nc[e], WD);
+                b[2 * u + e][m] = SUBS > 1 ? r[e] + nc[e] : r[e];
+            }
+        }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int o = WD; o < 4; o <<= 1) cabs[u] += __shfl_xor_sync(0xffffffffu, cabs[u], o);
+    // solve, test, store: the lanes of a group take its components in turn
+    bool flag = false;
+    float out[4][DIM];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (SUBS > 1 && u % SUBS != sub) continue;
+        const bool here = mine && c0 + u < g.nf;
+        const bool f = g1_solve<DIM>(L, b[u], cabs[u], cond, hinv, out[u]);
+        flag |= here && f;
+        float *o1 = g.d1 + (orow * g.nf + c0 + u) * DIM;
+#pragma unroll
+        for (int m = 0; m < DIM; ++m)  // (whole groups of a 3-D row are stored below)
+            if (here && (SUBS > 1 || DIM != 3 || !g.vec_d1)) o1[m] = out[u][m];
+    }
+    if (SUBS == 1 && DIM == 3 && g.vec_d1 && mine) {
+        float4 *o = reinterpret_cast<float4 *>(g.d1 + (orow * g.nf + c0) * 3);  // 48 bytes, 16-byte aligned
+        o[0] = make_float4(out[0][0], out[0][1 % DIM], out[0][2 % DIM], out[1][0]);
+        o[1] = make_float4(out[1][1 % DIM], out[1][2 % DIM], out[2][0], out[2][1 % DIM]);
+        o[2] = make_float4(out[2][2 % DIM], out[3][0], out[3][1 % DIM], out[3][2 % DIM]);
+    }
+    return flag;
+}
+
+template <int DIM>
+__global__ __launch_bounds__(128, 6) void k_grad1(GradArgs g) {
+    constexpr int NM = DIM * (DIM + 1) / 2;
+    extern __shared__ __align__(16) unsigned char g1_smem[];
+    G1Smem S;
+    S.wx = reinterpret_cast<float4 *>(g1_smem);
+    S.s = reinterpret_cast<int32_t *>(S.wx + g.k * kG1Queries);
+    const int ql = threadIdx.x >> 2, gl = threadIdx.x & 3;
+    const int64_t q0 = blockIdx.x * (int64_t)kG1Queries + ql;
+    const bool valid = q0 < g.nq;
+    const int64_t q = valid ? q0 : g.nq - 1;  // the lanes past the last query shadow it
+    const int32_t p = g.queries ? g.queries[q] : (int32_t)q;
+    const float4 h0 = g.hi[p], l0 = g.lo[p];
+    const ff hinv = ff_recip2(g.hsml[q], g.hsml_lo ? g.hsml_lo[q] : 0.0f);
+    float M[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) M[i] = 0.0f;
+    const int32_t *nb = g.ngb + q * g.k;
+    auto neighbour = [&](int j, int32_t s) {
+        float x[3];
+        const float w = g1_neighbour<DIM>(g, h0, l0, hinv, s, x);
+        float wx[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) wx[a] = w * x[a];
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int jj = 0; jj <= i; ++jj) M[i * (i + 1) / 2 + jj] += wx[i] * x[jj];
+        S.wx[g1_at(j, ql)] = make_float4(wx[0], wx[1], wx[2], w);
+        S.s[g1_at(j, ql)] = s;
+    };
+    // neighbouring entries of a row on neighbouring lanes: a row lists mostly
+    // ascending slots, so that the four lanes often read one line
+#pragma unroll 4
+    for (int j = gl; j < g.k; j += 4) neighbour(j, __ldg(nb + j));
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        M[i] += __shfl_xor_sync(0xffffffffu, M[i], 1);
+        M[i] += __shfl_xor_sync(0xffffffffu, M[i], 2);
+    }
+    __syncwarp();  // a query's lanes are in one warp
+    float L[NM], cond;
+    bool flag = g1_factor<DIM>(g, h0, hinv.hi, M, L, cond);
+    const int64_t orow = g.out_rows ? (int64_t)g.out_rows[q] : q;
+    const int ng = g.nfp >> 2;
+    for (int gr = 0; gr < ng;) {
+        const int rem = ng - gr;
+        if (rem >= 3) {
+            flag |= g1_fields<DIM, 4>(g, S, gr, ng, ql, gl, p, orow, valid, L, hinv.hi, cond);
+            gr += 4;
+        } else if (rem == 2) {
+            flag |= g1_fields<DIM, 2>(g, S, gr, ng, ql, gl, p, orow, valid, L, hinv.hi, cond);
+            gr += 2;
+        } else {
+            flag |= g1_fields<DIM, 1>(g, S, gr, ng, ql, gl, p, orow, valid, L, hinv.hi, cond);
+            gr += 1;
+        }
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, flag) >> (threadIdx.x & 28) & 0xfu;
+    if (any && gl == 0 && valid && g.fix_queue) g.fix_queue[atomicAdd(g.fix_count, 1)] = (int32_t)q;
+}
+
 // ---- FP64 re-solve of queued (ill-conditioned or singular) rows ------------------
 // Follows the reference arithmetic: FP64 separations from the FP64 positions,
 // FP64 kernel weights and moment sums (src/meshoid/derivatives.py:27-103).
@@ -587,28 +831,29 @@ template <int DIM, int ORDER>
 static int launch_grad(const GradArgs &g0, cudaStream_t st) {
     GradArgs g = g0;
     const unsigned blocks = (unsigned)((g.nq + 127) / 128);
-    // Components per launch: up to 8 (order 1) or 4 (order 2), as many as the
-    // registers hold with the compensated sums.  A launch with NF components
-    // reads columns [c0, c0 + NF) of rows of stride nfp, so NF never exceeds
-    // nfp - c0 (both multiples of 4).
-    for (int c0 = 0; c0 < g.nfp;) {
-        g.c0 = c0;
-        const int rem = g.nfp - c0;
-        int nf_launch = 4;
-        if constexpr (ORDER == 1) {
-            if (MG_GRAD_NF8 && rem >= 8) {
-                k_grad<DIM, ORDER, 8><<<blocks, 128, 0, st>>>(g);
-                nf_launch = 8;
-            } else {
-                k_grad<DIM, ORDER, 4><<<blocks, 128, 0, st>>>(g);
-            }
-        } else if (g.refine) {
-            k_grad<DIM, ORDER, 4, true><<<blocks, 128, 0, st>>>(g);
-        } else {
+    if constexpr (ORDER == 1) {
+        // results of nf a multiple of 4 keep the alignment of their first element
+        g.vec_d1 = (g.nf & 3) == 0 && ((uintptr_t)g.d1 & 15) == 0;
+        if (g.nfp == 4) {
             k_grad<DIM, ORDER, 4><<<blocks, 128, 0, st>>>(g);
+        } else if (g.nfp == 8) {
+            k_grad<DIM, ORDER, 8><<<blocks, 128, 0, st>>>(g);
+        } else {
+            const size_t smem = (size_t)g.k * kG1Queries * (sizeof(float4) + sizeof(int32_t));
+            MG_CUDA(cudaFuncSetAttribute(k_grad1<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_grad1<DIM><<<(unsigned)((g.nq + kG1Queries - 1) / kG1Queries), 128, smem, st>>>(g);
         }
         MG_CHECK_LAUNCH();
-        c0 += nf_launch;
+    } else {
+        // 4 components per launch, as many as the registers hold with the
+        // compensated sums
+        for (g.c0 = 0; g.c0 < g.nfp; g.c0 += 4) {
+            if (g.refine)
+                k_grad<DIM, ORDER, 4, true><<<blocks, 128, 0, st>>>(g);
+            else
+                k_grad<DIM, ORDER, 4><<<blocks, 128, 0, st>>>(g);
+            MG_CHECK_LAUNCH();
+        }
     }
     if (g.fix_queue) {
         int dev = 0, nsm = 148;

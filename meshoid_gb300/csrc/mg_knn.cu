@@ -32,6 +32,7 @@
 #include <cfloat>
 
 #include "mg_common.cuh"
+#include "mg_f32x2.cuh"
 #include "mg_grad2.cuh"
 #include "mg_hsml.cuh"
 #include "mg_refine.cuh"
@@ -1817,29 +1818,6 @@ __device__ __forceinline__ float group_d2(float cx, float cy, float cz, float qx
         d2 = __fmaf_rn(dz, dz, d2);
     }
     return d2;
-}
-
-// Two FP32 lanes in one 64-bit register (element 0 in the low half), with the
-// packed arithmetic of sm_100+: each half rounds as the scalar instruction.
-__device__ __forceinline__ unsigned long long f2_pack(float v) {
-    const unsigned long long b = __float_as_uint(v);
-    return b | (b << 32);
-}
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
 }
 
 // Optional phase cycle counters of the first pass (build with
