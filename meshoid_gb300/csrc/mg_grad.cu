@@ -827,6 +827,174 @@ __global__ __launch_bounds__(128) void k_grad_fix(GradArgs g) {
     }
 }
 
+// Order 1: four lanes per row, eight rows per block of one warp.  The lanes split
+// the neighbours; w x of each waits in shared memory in FP64, so that it is
+// computed once whatever the number of components.  Bound: the FP64 pipe (~2
+// lanes per cycle and SM) and, with the few rows there are, latency: one thread
+// per row, in blocks of 128 that left most SMs idle, recomputed the basis for
+// every 8 components.  10^6 Plummer particles with 16 components (~5,000 rows):
+// 0.29 -> 0.08 ms; 2^22 clumped with 19: the sweep 3.9 -> 3.65 ms.
+constexpr int kFixRows = 8;
+
+template <int DIM>
+__global__ __launch_bounds__(32) void k_grad_fix1(GradArgs g) {
+    extern __shared__ __align__(16) unsigned char fix_smem[];
+    double *S = reinterpret_cast<double *>(fix_smem);  // [neighbour][row][DIM]
+    const int gl = threadIdx.x & 3, rl = threadIdx.x >> 2;
+    const int nfix = *g.fix_count;
+    for (int e0 = blockIdx.x * kFixRows; e0 < nfix; e0 += gridDim.x * kFixRows) {
+        const bool valid = e0 + rl < nfix;
+        const int64_t q = g.fix_queue[valid ? e0 + rl : e0];  // the lanes past the last row shadow the first
+        const int32_t p = g.queries ? g.queries[q] : (int32_t)q;
+        const double h = (double)g.hsml[q] + (g.hsml_lo ? (double)g.hsml_lo[q] : 0.0), hinv = 1.0 / h;
+        const int32_t *nb = g.ngb + q * g.k;
+        double A[DIM][DIM];
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) A[i][j] = 0.0;
+        double p0[DIM];
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) p0[c] = g.pos64[(int64_t)p * 3 + c];
+        for (int j = gl; j < g.k; j += 4) {
+            const int32_t s = nb[j];
+            double x[DIM], r2 = 0.0;
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) {
+                double d = g.pos64[(int64_t)s * 3 + c] - p0[c];
+                if (g.periodic && fabs(d) > 0.5 * g.box) d = -copysign(g.box - fabs(d), d);
+                x[c] = d * hinv;
+                r2 += x[c] * x[c];
+            }
+            double w = 1.0;
+            if (g.weighted) {
+                const double qq = sqrt(r2);
+                w = qq <= 0.5 ? 1.0 - 6.0 * qq * qq + 6.0 * qq * qq * qq
+                              : (qq <= 1.0 ? 2.0 * (1.0 - qq) * (1.0 - qq) * (1.0 - qq) : 0.0);
+            }
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) {
+                const double wa = w * x[i];
+                S[(j * kFixRows + rl) * DIM + i] = wa;
+#pragma unroll
+                for (int jj = 0; jj <= i; ++jj) A[i][jj] += wa * x[jj];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int jj = 0; jj <= i; ++jj) {
+                A[i][jj] += __shfl_xor_sync(0xffffffffu, A[i][jj], 1);
+                A[i][jj] += __shfl_xor_sync(0xffffffffu, A[i][jj], 2);
+                A[jj][i] = A[i][jj];
+            }
+        __syncwarp();
+        // inverse (Cholesky-based when positive definite, pseudo-inverse otherwise)
+        double P[DIM][DIM];
+        bool spd = true;
+        {
+            double Lc[DIM][DIM], inv[DIM];
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) {
+                double sd = A[j][j];
+#pragma unroll
+                for (int k2 = 0; k2 < j; ++k2) sd -= Lc[j][k2] * Lc[j][k2];
+                spd = spd && sd > 1e-14 * fmax(A[0][0], 1e-300);
+                const double d = sqrt(spd ? sd : 1.0);
+                Lc[j][j] = d;
+                inv[j] = 1.0 / d;
+#pragma unroll
+                for (int i = j + 1; i < DIM; ++i) {
+                    double t = A[i][j];
+#pragma unroll
+                    for (int k2 = 0; k2 < j; ++k2) t -= Lc[i][k2] * Lc[j][k2];
+                    Lc[i][j] = t * inv[j];
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) {
+                double x[DIM];
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) {
+                    double t = i == c ? 1.0 : 0.0;
+#pragma unroll
+                    for (int k2 = 0; k2 < i; ++k2) t -= Lc[i][k2] * x[k2];
+                    x[i] = t * inv[i];
+                }
+#pragma unroll
+                for (int i = DIM - 1; i >= 0; --i) {
+                    double t = x[i];
+#pragma unroll
+                    for (int k2 = i + 1; k2 < DIM; ++k2) t -= Lc[k2][i] * x[k2];
+                    x[i] = t * inv[i];
+                }
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) P[i][c] = x[i];
+            }
+        }
+        if (!spd) jacobi_pinv<DIM>(A, P);
+        if (valid && gl == 0 && g.qstatus) atomicOr(g.qstatus + q, MG_Q_FP64_SOLVE | (spd ? 0 : MG_Q_SINGULAR));
+        const int64_t orow = g.out_rows ? (int64_t)g.out_rows[q] : q;
+        auto sum = [](float hi, float lo) -> double { return (double)hi + (double)lo; };
+        for (int c0 = 0; c0 < g.nf; c0 += 4) {
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 gh = *reinterpret_cast<const float4 *>(g.f_hi + (int64_t)p * g.nfp + c0);
+            const float4 gw = g.f_lo ? *reinterpret_cast<const float4 *>(g.f_lo + (int64_t)p * g.nfp + c0) : zero;
+            const double f0[4] = {sum(gh.x, gw.x), sum(gh.y, gw.y), sum(gh.z, gw.z), sum(gh.w, gw.w)};
+            double b[4][DIM];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) b[u][i] = 0.0;
+#pragma unroll 2
+            for (int j = gl; j < g.k; j += 4) {
+                const int32_t s = nb[j];
+                const float4 vh = *reinterpret_cast<const float4 *>(g.f_hi + (int64_t)s * g.nfp + c0);
+                const float4 vl = g.f_lo ? *reinterpret_cast<const float4 *>(g.f_lo + (int64_t)s * g.nfp + c0) : zero;
+                const double df[4] = {sum(vh.x, vl.x) - f0[0], sum(vh.y, vl.y) - f0[1], sum(vh.z, vl.z) - f0[2],
+                                      sum(vh.w, vl.w) - f0[3]};
+                double wa[DIM];
+                long long some = 0;
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) {
+                    wa[i] = S[(j * kFixRows + rl) * DIM + i];
+                    some |= __double_as_longlong(wa[i]);
+                }
+                if (some << 1 == 0) continue;  // no weight: whatever its field, infinite or NaN too
+#pragma unroll
+                for (int i = 0; i < DIM; ++i)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (c0 + u < g.nf) b[u][i] += wa[i] * df[u];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c0 + u >= g.nf) break;
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) {
+                    b[u][i] += __shfl_xor_sync(0xffffffffu, b[u][i], 1);
+                    b[u][i] += __shfl_xor_sync(0xffffffffu, b[u][i], 2);
+                }
+            }
+            // lane u solves and stores component c0 + u
+            double bb[DIM];
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) bb[i] = gl == 0 ? b[0][i] : (gl == 1 ? b[1][i] : (gl == 2 ? b[2][i] : b[3][i]));
+            if (valid && c0 + gl < g.nf) {
+                float *o1 = g.d1 + (orow * g.nf + c0 + gl) * DIM;
+#pragma unroll
+                for (int m = 0; m < DIM; ++m) {
+                    double t = 0.0;
+#pragma unroll
+                    for (int i = 0; i < DIM; ++i) t += P[m][i] * bb[i];
+                    o1[m] = (float)(t * hinv);
+                }
+            }
+        }
+        __syncwarp();  // the row's w x are rewritten
+    }
+}
+
 template <int DIM, int ORDER>
 static int launch_grad(const GradArgs &g0, cudaStream_t st) {
     GradArgs g = g0;
@@ -859,9 +1027,16 @@ static int launch_grad(const GradArgs &g0, cudaStream_t st) {
         int dev = 0, nsm = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const int64_t want = (g.nq + 127) / 128;
-        const unsigned fb = (unsigned)(want < (int64_t)nsm * 4 ? want : (int64_t)nsm * 4);
-        k_grad_fix<DIM, ORDER><<<fb, 128, 0, st>>>(g);
+        if constexpr (ORDER == 1) {
+            const int64_t want = (g.nq + kFixRows - 1) / kFixRows;
+            const unsigned fb = (unsigned)(want < (int64_t)nsm * 16 ? want : (int64_t)nsm * 16);
+            const size_t smem = (size_t)g.k * kFixRows * DIM * sizeof(double);
+            k_grad_fix1<DIM><<<fb, 32, smem, st>>>(g);  // 24 KB at MG_MAX_K
+        } else {
+            const int64_t want = (g.nq + 127) / 128;
+            const unsigned fb = (unsigned)(want < (int64_t)nsm * 4 ? want : (int64_t)nsm * 4);
+            k_grad_fix<DIM, ORDER><<<fb, 128, 0, st>>>(g);
+        }
         MG_CHECK_LAUNCH();
     }
     return MG_OK;
