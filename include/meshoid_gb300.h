@@ -165,8 +165,8 @@ size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k);
  *   seed_h: nq FP32 first guesses of h; the first search radius is
  *           radius_factor * seed_h.  A query whose radius holds fewer than k
  *           particles (or too many) is searched again with a corrected
- *           radius, up to 4 max_passes times (max_passes 1: once; k > 32: in
- *           up to max_passes passes).
+ *           radius, up to 4 max_passes times (max_passes 1: once; k > 32 and
+ *           query lists: in up to max_passes passes).
  *   level_bias: 0 or 1 -- the searched cells have side >= R / 2^level_bias
  *           (finer cells: fewer candidates, more cell lookups).
  *   ngb:    nq * k slots, unordered within a row (the set is exact: the k
@@ -178,13 +178,14 @@ size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k);
  *           with mg_hsml_polish).  hsml alone is good to ~1e-7.
  *           qstatus: nq MG_Q_* bits.
  *   stats:  16 int64 device counters, accumulated (the caller zeroes them):
- *           [0] most searches any query took after its first in the warp
- *           path (k > 32: passes after the first), [1] candidates scanned (warp path) or staged (first pass,
- *           per query it serves), [2] retries, [3] FP64 band re-decisions,
- *           [4] unresolved, [5] Newton steps, [6..8] retries for too few /
- *           too many / band outside the radius, [9] scan lists narrowed
- *           before the scan, or for k > 32 handed to a block (crowded: a
- *           sparse query beside a dense clump).
+ *           [0] most searches any query took after its first in the warp path
+ *           (k > 32 and query lists: passes after the first), [1] candidates
+ *           scanned (warp path) or streamed or staged (first pass, per query
+ *           it serves), [2] retries, [3] FP64 band re-decisions, [4]
+ *           unresolved, [5] Newton steps, [6..8] retries for too few / too
+ *           many / band outside the radius, [9] crowded scan lists (a sparse
+ *           query beside a dense clump) narrowed before the scan, or handed
+ *           to a block (k > 32 and query lists).
  * Replaces tree.query + HsmlIter (src/meshoid/Meshoid.py:157,165;
  * src/meshoid/kernel_density.py:15-56). */
 int mg_knn_hsml(const mg_cells *cells, const int32_t *queries, int64_t nq, int32_t k,
@@ -193,9 +194,9 @@ int mg_knn_hsml(const mg_cells *cells, const int32_t *queries, int64_t nq, int32
                 float *hsml, float *hsml_lo, int32_t *qstatus, int64_t *stats, void *workspace,
                 size_t workspace_bytes, void *stream);
 /* First pass of mg_knn_hsml: 1 (default) runs it one thread per query over
- * candidates staged once per block of 128 consecutive queries, the queries it
- * cannot decide exactly going on to the warp-per-query path; 0 runs every
- * query there.  Both give the same neighbour sets and distances.
+ * the candidates streamed for its warp's 32 consecutive queries (k <= 32), the
+ * queries it cannot decide exactly going on to the warp-per-query path; 0 runs
+ * every query there.  Both give the same neighbour sets and distances.
  * Process-wide; returns the previous setting. */
 int mg_knn_set_group_pass(int32_t enabled);
 /* Kept for its callers: the warp path of mg_knn_hsml is one launch of

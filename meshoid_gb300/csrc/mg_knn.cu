@@ -4,11 +4,11 @@
 // Replaces cKDTree.query(pos[mask], des_ngb) (src/meshoid/Meshoid.py:157)
 // followed by HsmlIter (src/meshoid/kernel_density.py:15-56).
 //
-// Search, first pass (k_knn_group): one thread per query over the particles
-// staged once per block of 128 consecutive queries; it accepts a query only
-// when an error bound proves its set exact, and queues the rest.
+// Search, first pass (k_knn_group, k <= 32): one thread per query over the
+// particles streamed once for its warp of 32 consecutive queries; it accepts a
+// query only when an error bound proves its set exact, and queues the rest.
 //
-// Search, warp path (k_knn_hsml; every query for periodic boxes or k > 32):
+// Search, warp path (k_knn_hsml; for k > 32 every query, in k_knn_pass):
 // the query's radius R comes from a seed or the queue.  The level L with cell
 // side s_L >= R (or R / 2) is chosen, the level-L cells that meet the sphere
 // of radius R are looked up (dense table for L <= grid_level, refinement
@@ -71,7 +71,7 @@ constexpr int kNarrowCell = 48;  // cells of up to this many particles are not s
 // them all, so that a warp reuses its cell box.
 constexpr unsigned kRun = 8;
 
-// Passes over the queue for k > 32 (k_knn_pass, k_knn_heavy)
+// Passes over the queue (k_knn_pass, k_knn_heavy)
 constexpr int kChunk = 32;     // consecutive queries per warp on the first pass
 constexpr int kSplit = 192;    // cells holding more particles than this are split when they straddle the sphere
 constexpr int kHeavy = 2048;   // scan-list particles above which a query goes to the block-wide path
@@ -732,15 +732,16 @@ __device__ KNN_SELECT_INLINE void finish_row(SM &S, int cnt, float T, int k, int
     }
 }
 
-// ---- k > 32: passes over a queue -------------------------------------------------
+// ---- k > 32 and query lists: passes over a queue ----------------------------------
 // For k > 32 h is solved in FP32 from the row's distances in the row's order,
 // so that the order of a row, which follows from how its query was searched,
-// shows in h and the density at ~3e-8.  These rows keep the search that
-// produced them so far, and with it every bit of their results: a pass of
-// warps over the queue (k_knn_pass), then a block per crowded query
-// (k_knn_heavy), undecided queries queued for the next pass.  For k <= 32 h is
-// solved in float-float, where the order does not show above 1e-13, and
-// k_knn_hsml decides every query in place.
+// shows in h and the density at ~3e-8; and the FP64 values that Slice and
+// Reconstruct build on the derivatives of a query list show it at ~1e-8.  These
+// rows keep the search that produced them so far, and with it every bit of
+// their results: a pass of warps over the queue (k_knn_pass), then a block per
+// crowded query (k_knn_heavy), undecided queries queued for the next pass.  For
+// k <= 32 h is solved in float-float, where the order does not show above
+// 1e-13, and over a full set k_knn_hsml decides every query in place.
 // Rare path (out of line): entries of the scan-list chunk starting at i0 that
 // hold more than kSplit particles and straddle the sphere are replaced by their
 // non-empty children that meet it (open 3-D boxes; children of a level-l cell
@@ -1739,7 +1740,568 @@ __global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_hsml(cons
     }
 }
 
-// ---- first pass, one thread per query over a block-shared candidate set --------
+// ---- first pass, one thread per query over a warp's candidates -----------------
+// The 32 queries of a warp are consecutive (neighbours in Morton order).  The
+// warp takes the boxes of each eight queries' first-radius spheres (queries whose
+// radius is over kGroupOutlier times the warp's smallest are left to the warp
+// path), looks up the cells over them as runs of consecutive slots, and streams
+// those particles: 128 are loaded at a time, the ones inside the common box are
+// staged in shared memory as offsets from its centre (FP32), and every lane
+// tests them against its
+// own query and lists those with d~ <= R as one word: d~^2 / R^2 in 20 bits and
+// the particle's place in the stream in 12.  Each lane then selects from its
+// list: two passes count it in 8 and 8 x 8 buckets of d~^2 and a third takes
+// those below the k-th neighbour's bucket and sets its bucket aside, whose
+// smallest are taken one by one.
+//
+// d~ differs from the distance by at most e (a bound from the box size, and half
+// a unit of the 20 bits), so the set is the exact k nearest when the k-th d~
+// plus e stays inside R (every particle that is not listed is farther than R)
+// and the next d~ is more than 2e beyond the k-th.  Every other query (too few
+// in radius, a near tie, a crowded bucket, a full list, a box over too many
+// particles) goes to the work queue, and the warp path finishes it.  Only the
+// rows' slots are written, in stream order; h is solved from them by
+// k_hsml_solve_rows with the warp path's FP32 hi/lo distances (cand_d2p).
+//
+// Nothing is shared between warps: no block barrier, and no buffer whose overflow
+// sends a block's queries away.  Staging once for 128 queries, with barriers
+// between its rounds, held 12 warps per SM at 40% issue and left 7% of the
+// queries to the warp path; here 14 warps issue on ~60% of the cycles.  2^22
+// Plummer particles, first pass 7.33 -> 3.3 ms, warp path 1.74 -> 1.0 ms; 2^24
+// clump mixture 29.0 -> 14 and 11.6 -> 7 ms.  Bound: instruction issue: testing
+// the ~700 particles in the box against each query (a third), streaming ~1700 to
+// find them (a quarter), the selection (a fifth).
+constexpr int kGroupWarps = 2;      // warps per block (independent of each other)
+constexpr int kGroupRuns = 128;     // runs of slots per warp
+constexpr int kGroupStream = 4096;  // particles a warp streams at most (12 bits)
+// Listed candidates per query: 16.5 KB per warp, 14 warps per SM.  88 and 104
+// entries: 3% and 4% slower on 2^22 Plummer particles (more queries left to the
+// warp path; fewer warps); lists cut back to their k nearest when full instead:
+// 80 to 88 entries, 7% slower (the check in the inner loop).
+constexpr int kGroupList = 96;
+constexpr int kGroupBoundary = 8;   // entries of the k-th neighbour's bucket
+constexpr int kGroupUnroll = 4;     // chunks of 32 particles loaded together
+constexpr int kGroupBoxes = 4;      // boxes per warp, of eight queries each
+#ifndef MG_KNN_GROUP_OUTLIER
+#define MG_KNN_GROUP_OUTLIER 2.0f
+#endif
+constexpr float kGroupOutlier = MG_KNN_GROUP_OUTLIER;  // radius above this multiple of the warp's smallest: warp path
+
+struct GroupSmem {  // per warp
+    static constexpr int kStage = 32 * kGroupUnroll + 4;
+    float sx[kStage], sy[kStage], sz[kStage];  // staged: offsets from the box centre
+    uint32_t sg[kStage];                       // and place in the stream
+    // entry e of lane t at 32 e + t: one bank per lane, whatever the entries.  The
+    // k-th neighbours' buckets take the staging arrays once the stream is done.
+    uint32_t list[32 * kGroupList];
+    uint32_t pa[kGroupRuns];      // first slot of each run
+    uint32_t off[kGroupRuns + 4]; // prefix offsets of the runs in the stream
+    int cells[kGroupBoxes][6];    // cells over each box: first x y z, last x y z
+};
+
+// First slots of the eight children (level L) of the level L - 1 cell `code`
+// where a table holds them: child i starts at p[i << sh], i up to 8.  Without a
+// table (a cell of few particles, or no refinement tables): false, and [A, B)
+// is the range of the smallest tabled cell around it.
+__device__ __forceinline__ bool child_table(const CellIndex &ci, int L, uint64_t code, const uint32_t *&p, int &sh,
+                                            uint32_t &A, uint32_t &B) {
+    if (L <= ci.Lg) {
+        sh = 3 * (ci.Lg - L);
+        p = ci.cs + ((code << 3) << sh);
+        return true;
+    }
+    const uint64_t c = code >> (3 * (L - 1 - ci.Lg));
+    A = __ldg(ci.cs + c);
+    B = __ldg(ci.cs + c + 1);
+    int br = ci.brick_of ? __ldg(ci.brick_of + c) : -1;
+    int base = ci.Lg;
+    while (br >= 0) {
+        const uint32_t *st = ci.bricks + (size_t)br * kBrickWords;
+        if (L <= base + 3) {
+            sh = 3 * (base + 3 - L);
+            p = st + ((uint32_t)((code & ((1ull << (3 * (L - 1 - base))) - 1ull)) << 3) << sh);
+            return true;
+        }
+        const uint32_t sub = (uint32_t)((code >> (3 * (L - 1 - base - 3))) & 511ull);
+        A = __ldg(st + sub);
+        B = __ldg(st + sub + 1);
+        br = (int)__ldg(st + kBrickChild + sub);
+        base += 3;
+    }
+    return false;
+}
+
+// Offset of a position (hi, lo) from the box centre: its nearest image when
+// periodic, the wrap carried error-free (wrap1's form).
+template <bool PERIODIC>
+__device__ __forceinline__ float group_offset(float h, float l, float c, float box_hi, float box_lo) {
+    if (!PERIODIC) return __fadd_rn(__fsub_rn(h, c), l);
+    float s, e;
+    two_sum(h, -c, s, e);
+    if (fabsf(s) > 0.5f * box_hi) {
+        const float sg = s > 0.0f ? 1.0f : -1.0f;
+        float s2, e2;
+        two_sum(s, -sg * box_hi, s2, e2);
+        return s2 + ((e2 + e + l) - sg * box_lo);
+    }
+    return s + (e + l);
+}
+
+// The byte (0 to 7) of the packed counts at which their running sum from `below`
+// reaches k; below: the sum before it, in: its count.
+__device__ __forceinline__ int group_bucket(unsigned long long counts, int k, int &below, int &in) {
+    int b = 7;
+    bool found = false;
+    int run = below, at = below, n = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int c = (int)(counts >> (8 * i)) & 255;
+        const bool here = !found && run + c >= k;
+        b = here ? i : b;
+        at = here ? run : at;
+        n = here ? c : n;
+        found = found || here;
+        run += c;
+    }
+    below = at;
+    in = n;
+    return b;
+}
+
+template <int DIM, bool PERIODIC>
+__global__ __launch_bounds__(32 * kGroupWarps, 7) void k_knn_group(const __grid_constant__ KnnArgs a) {
+    extern __shared__ __align__(16) unsigned char group_smem[];
+    GroupSmem &S = reinterpret_cast<GroupSmem *>(group_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t qi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool valid = qi < a.nq;
+    const Frame fr = load_frame(a.frame);
+    const float side = (float)fr.side;
+    const float half_side = 0.5f * side;
+    const int k = a.k;
+
+    float4 h0 = make_float4(0.f, 0.f, 0.f, 0.f), l0 = h0;
+    float R = 0.0f;
+    if (valid) {
+        const int32_t p = a.queries ? a.queries[qi] : (int32_t)qi;
+        h0 = a.hi[p];
+        l0 = a.lo[p];
+        R = a.seed_h[qi] * a.radius_factor;
+        if (!(R > 0.0f) || !isfinite(R)) R = side * 1e-3f;
+    }
+    // ---- members and their box (hi parts) ----------------------------------------
+    const float rmin = warp_min(valid ? R : FLT_MAX);
+    const bool mine = valid && R <= kGroupOutlier * rmin;
+    float blo[3] = {0.0f, 0.0f, 0.0f}, bhi[3] = {0.0f, 0.0f, 0.0f};
+    {
+        const float h[3] = {h0.x, h0.y, h0.z};
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            blo[d] = warp_min(mine ? h[d] - R : FLT_MAX);
+            bhi[d] = -warp_min(mine ? -(h[d] + R) : FLT_MAX);
+        }
+    }
+    const float rmax = -warp_min(mine ? -R : FLT_MAX);
+    // the hi parts differ from the positions by up to 2^-24 |x|
+    float xm = 0.0f;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xm = fmaxf(xm, fmaxf(fabsf(blo[d]), fabsf(bhi[d])));
+    if (PERIODIC) xm = fmaxf(xm, a.box_hi);
+    const float mg = 1e-5f * rmax + 4e-7f * xm + 1e-30f;
+    float ctr[3] = {0.0f, 0.0f, 0.0f}, ext = 0.0f, ehalf = 0.0f;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        blo[d] -= mg;
+        bhi[d] += mg;
+        ctr[d] = 0.5f * (blo[d] + bhi[d]);
+        ext = fmaxf(ext, bhi[d] - blo[d]);
+        ehalf = fmaxf(ehalf, fmaxf(fabsf(blo[d] - ctr[d]), fabsf(bhi[d] - ctr[d])));
+    }
+    // offsets from the centre carry at most ~2^-23 ehalf of rounding per axis,
+    // and the hi/lo split of each position ~2^-48 |x| of representation error
+    // (2^-46 |x| per axis for a difference, with the low parts' rounding):
+    // bound on |d~ - d| for d <= R (twice the analysis)
+    const float eg = 1e-6f * ehalf + 3e-7f * rmax + 3e-14f * xm;
+    float qx = 0.0f, qy = 0.0f, qz = 0.0f;
+    qx = __fadd_rn(__fsub_rn(h0.x, ctr[0]), l0.x);
+    if (DIM > 1) qy = __fadd_rn(__fsub_rn(h0.y, ctr[1]), l0.y);
+    if (DIM > 2) qz = __fadd_rn(__fsub_rn(h0.z, ctr[2]), l0.z);
+    // box of the member spheres, and those of each eight queries (lanes 8 b ..
+    // 8 b + 7), in offsets
+    float qlo[3], qhi[3];  // of all
+    float elo[3], ehi[3];  // of this lane's eight
+    {
+        const float rr = R * (1.0f + 1e-6f) + eg;
+        const float qv[3] = {qx, qy, qz};
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            elo[d] = mine ? qv[d] - rr : FLT_MAX;
+            ehi[d] = mine ? qv[d] + rr : -FLT_MAX;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                elo[d] = fminf(elo[d], __shfl_xor_sync(0xffffffffu, elo[d], o));
+                ehi[d] = fmaxf(ehi[d], __shfl_xor_sync(0xffffffffu, ehi[d], o));
+            }
+            qlo[d] = elo[d];
+            qhi[d] = ehi[d];
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) {
+                qlo[d] = fminf(qlo[d], __shfl_xor_sync(0xffffffffu, qlo[d], o));
+                qhi[d] = fmaxf(qhi[d], __shfl_xor_sync(0xffffffffu, qhi[d], o));
+            }
+        }
+    }
+    // ---- cells over the box: finest level with at most 8 per axis -----------------
+    int L = (int)floorf(log2f(side / ext)) + 3;
+    L = max(1, min(kMaxLevel, L));
+    int cmin[3] = {0, 0, 0}, cmax[3] = {0, 0, 0};
+    bool ok = rmin < FLT_MAX;
+    for (;;) {
+        const float cps = (float)(1u << L), scale = cps / side;
+        const float em = 1e-3f + cps * 2.4e-7f;
+        bool fits = true;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            cmin[d] = (int)floorf((blo[d] + half_side) * scale - em);
+            cmax[d] = (int)floorf((bhi[d] + half_side) * scale + em);
+            if (!PERIODIC) {
+                cmin[d] = max(0, cmin[d]);
+                cmax[d] = min((int)cps - 1, cmax[d]);
+            }
+            fits = fits && cmax[d] - cmin[d] < 8;
+        }
+        if (fits) break;
+        if (L == 1) {
+            ok = false;
+            break;
+        }
+        --L;
+    }
+    if ((lane & 7) == 0) {  // (an empty box: no cell)
+        const float cps = (float)(1u << L), scale = cps / side;
+        const float em = 1e-3f + cps * 2.4e-7f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const bool some = d < DIM && elo[d < DIM ? d : 0] <= ehi[d < DIM ? d : 0];
+            const float c0 = d < DIM ? (elo[d] + ctr[d] - mg + half_side) * scale - em : 0.0f;
+            const float c1 = d < DIM ? (ehi[d] + ctr[d] + mg + half_side) * scale + em : 0.0f;
+            S.cells[lane >> 3][d] = some ? max(cmin[d], (int)floorf(c0)) : (d < DIM ? INT_MAX : 0);
+            S.cells[lane >> 3][3 + d] = some ? min(cmax[d], (int)floorf(c1)) : (d < DIM ? INT_MIN : 0);
+        }
+    }
+    __syncwarp();
+    // a box of nearly the period's size: images would be ambiguous, cells repeat
+    if (PERIODIC) ok = ok && ext < 0.4f * a.box_hi && L >= 4;
+    // ---- runs of consecutive slots under those cells --------------------------------
+    int nrun = 0, tot = 0;
+    if (ok) {
+        int pmin[3], pn[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            pmin[d] = cmin[d] >> 1;
+            pn[d] = (cmax[d] >> 1) - pmin[d] + 1;  // <= 5
+        }
+        const int npar = pn[0] * pn[1] * pn[2];
+        const float inv_nx = 1.0f / (float)pn[0], inv_nxy = 1.0f / (float)(pn[0] * pn[1]);
+        const int wrap = (1 << (L - 1)) - 1;
+        KNN_LOOP_HINT
+        for (int c0 = 0; c0 < npar; c0 += 32) {
+            const int c = c0 + lane;
+            const uint32_t *tp = nullptr;
+            int sh = 0;
+            unsigned m = 0;
+            uint32_t A = 0, B = 0;
+            if (c < npar) {
+                int ix, iy, iz;
+                box_index(c, inv_nx, inv_nxy, pn, ix, iy, iz);
+                const int X = pmin[0] + ix, Y = pmin[1] + iy, Z = pmin[2] + iz;
+                // children inside some box's cells
+#pragma unroll
+                for (int b = 0; b < kGroupBoxes; ++b) {
+                    const int *c = S.cells[b];
+                    const int x = 2 * X, y = 2 * Y, z = 2 * Z;
+                    unsigned mb = (x >= c[0] && x <= c[3] ? 0x55u : 0u) | (x + 1 >= c[0] && x < c[3] ? 0xaau : 0u);
+                    mb &= (y >= c[1] && y <= c[4] ? 0x33u : 0u) | (y + 1 >= c[1] && y < c[4] ? 0xccu : 0u);
+                    mb &= (z >= c[2] && z <= c[5] ? 0x0fu : 0u) | (z + 1 >= c[2] && z < c[5] ? 0xf0u : 0u);
+                    m |= mb;
+                }
+                const uint64_t code = morton3((uint32_t)(X & wrap), (uint32_t)(Y & wrap), (uint32_t)(Z & wrap));
+                if (m && !child_table(a.ci, L, code, tp, sh, A, B)) {
+                    const int ks = 3 * (kKeyBits - L + 1);
+                    A = lower_bound_prefix(a.keys, A, B, code, ks);
+                    B = lower_bound_prefix(a.keys, A, B, code + 1, ks);
+                    tp = nullptr;
+                    m = 1u;
+                }
+            }
+            while (__any_sync(0xffffffffu, m != 0u)) {
+                uint32_t ra = 0, rb = 0;
+                if (m) {
+                    const int i = __ffs(m) - 1, n = __ffs(~(m >> i)) - 1;  // children i .. i + n - 1
+                    ra = tp ? __ldg(tp + ((size_t)i << sh)) : A;
+                    rb = tp ? __ldg(tp + ((size_t)(i + n) << sh)) : B;
+                    m &= ~(((1u << n) - 1u) << i);
+                }
+                const int len = (int)(rb - ra);
+                const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+                const int pos = nrun + __popc(some & ((1u << lane) - 1u));
+                const int inc = warp_incl_scan(len);
+                if (len > 0 && pos < kGroupRuns) {
+                    S.pa[pos] = ra;
+                    S.off[pos] = (uint32_t)(tot + inc - len);
+                }
+                nrun += __popc(some);
+                tot += __shfl_sync(0xffffffffu, inc, 31);
+            }
+        }
+        ok = nrun <= kGroupRuns && tot <= kGroupStream && tot >= 0;
+        if (ok && lane == 0) S.off[nrun] = (uint32_t)tot;
+        __syncwarp();
+    }
+
+    // ---- stream: load, stage what lies in the box, list ------------------------------
+    // reason: 0 accepted, 1 too few in radius, 3 k-th too close to R, 4 other
+    const bool act = ok && mine;
+    const float R2 = R * R;
+    int cnt = 0;
+    bool full = false;
+    if (ok) {
+        // key of d~^2: its 20-bit fraction of R^2, read off the low mantissa bits
+        // of d~^2 s + 2^23
+        const float ks = 1048575.0f / R2;
+        float R2a = act ? R2 : -1.0f;
+        uint32_t *lp = S.list + lane;  // end of this lane's list
+        const uint32_t *const lp_full = lp + 32 * (kGroupList - 4);
+        const unsigned long long QX = f2_pack(qx), QY = f2_pack(qy), QZ = f2_pack(qz), KS = f2_pack(ks),
+                                 MAGIC = f2_pack(8388608.0f);
+        float4 hb[kGroupUnroll], lb[kGroupUnroll];
+        int j0 = 0;
+        auto fetch = [&](int g0) {
+            uint32_t slot[kGroupUnroll];
+#pragma unroll
+            for (int u = 0; u < kGroupUnroll; ++u) {
+                const int g = g0 + 32 * u;
+                slot[u] = g < tot ? chunk_slot(S, nrun, tot, g, j0, lane) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < kGroupUnroll; ++u) {
+                if (g0 + 32 * u + lane < tot) {
+                    hb[u] = __ldg(a.hi + slot[u]);
+                    lb[u] = __ldg(a.lo + slot[u]);
+                }
+            }
+        };
+        fetch(0);
+        KNN_LOOP_HINT
+        for (int g0 = 0; g0 < tot; g0 += 32 * kGroupUnroll) {
+            int n = 0;
+#pragma unroll
+            for (int u = 0; u < kGroupUnroll; ++u) {
+                const int g = g0 + 32 * u + lane;
+                const float ox = group_offset<PERIODIC>(hb[u].x, lb[u].x, ctr[0], a.box_hi, a.box_lo);
+                const float oy = DIM > 1 ? group_offset<PERIODIC>(hb[u].y, lb[u].y, ctr[1], a.box_hi, a.box_lo) : 0.0f;
+                const float oz = DIM > 2 ? group_offset<PERIODIC>(hb[u].z, lb[u].z, ctr[2], a.box_hi, a.box_lo) : 0.0f;
+                bool in = ox >= qlo[0] && ox <= qhi[0];
+                if (DIM > 1) in = in && oy >= qlo[1] && oy <= qhi[1];
+                if (DIM > 2) in = in && oz >= qlo[2] && oz <= qhi[2];
+                in = in && g < tot;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (in) {
+                    const int pos = n + __popc(m & ((1u << lane) - 1u));
+                    S.sx[pos] = ox;
+                    if (DIM > 1) S.sy[pos] = oy;
+                    if (DIM > 2) S.sz[pos] = oz;
+                    S.sg[pos] = (uint32_t)g;
+                }
+                n += __popc(m);
+            }
+            if (lane < 4) S.sx[n + lane] = 1e18f;  // pads the last four
+            if (g0 + 32 * kGroupUnroll < tot) fetch(g0 + 32 * kGroupUnroll);
+            __syncwarp();
+            KNN_LOOP_HINT
+            for (int w = 0; w < n; w += 4) {
+                const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(S.sx + w);
+                ulonglong2 Y, Z;
+                if (DIM > 1) Y = *reinterpret_cast<const ulonglong2 *>(S.sy + w);
+                if (DIM > 2) Z = *reinterpret_cast<const ulonglong2 *>(S.sz + w);
+                const uint4 G = *reinterpret_cast<const uint4 *>(S.sg + w);
+                R2a = lp > lp_full ? -1.0f : R2a;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const unsigned long long dx = f2_sub(h ? X.y : X.x, QX);
+                    unsigned long long d2 = f2_mul(dx, dx);
+                    if (DIM > 1) {
+                        const unsigned long long dy = f2_sub(h ? Y.y : Y.x, QY);
+                        d2 = f2_fma(dy, dy, d2);
+                    }
+                    if (DIM > 2) {
+                        const unsigned long long dz = f2_sub(h ? Z.y : Z.x, QZ);
+                        d2 = f2_fma(dz, dz, d2);
+                    }
+                    const unsigned long long t = f2_fma(d2, KS, MAGIC);
+                    const uint32_t k0 = (uint32_t)t * 4096u + (h ? G.z : G.x);
+                    const uint32_t k1 = (uint32_t)(t >> 32) * 4096u + (h ? G.w : G.y);
+                    if (f2_low(d2) <= R2a) {
+                        *lp = k0;
+                        lp += 32;
+                    }
+                    if (f2_high(d2) <= R2a) {
+                        *lp = k1;
+                        lp += 32;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        cnt = (int)(lp - (S.list + lane)) >> 5;
+        full = lp > lp_full;
+    }
+    // ---- per-lane selection ------------------------------------------------------------
+    int reason = 4;
+    float T = 0.0f;
+    if (act && !full) {
+        if (cnt < k) {
+            reason = 1;
+        } else {
+            unsigned long long c8 = 0ull;
+#pragma unroll 4
+            for (int e = 0; e < cnt; ++e) c8 += 1ull << ((S.list[32 * e + lane] >> 29) << 3);
+            int below = 0, in = 0;
+            const uint32_t b1 = (uint32_t)group_bucket(c8, k, below, in);
+            c8 = 0ull;
+#pragma unroll 4
+            for (int e = 0; e < cnt; ++e) {
+                const uint32_t v = S.list[32 * e + lane];
+                c8 += (v >> 29) == b1 ? 1ull << ((v >> 23) & 56u) : 0ull;
+            }
+            const uint32_t bstar = 8u * b1 + (uint32_t)group_bucket(c8, k, below, in);  // of 64
+            if (in <= kGroupBoundary) {
+                static_assert(32 * kGroupBoundary <= 2 * GroupSmem::kStage, "fits sx and sy");
+                uint32_t *bnd = reinterpret_cast<uint32_t *>(S.sx);
+                const int r = k - below;
+                int ns = 0, nb = 0;
+                uint32_t next = 0xffffffffu;  // smallest beyond the bucket
+#pragma unroll 4
+                for (int e = 0; e < cnt; ++e) {
+                    const uint32_t v = S.list[32 * e + lane], b = v >> 26;
+                    if (b < bstar) {
+                        S.list[32 * ns + lane] = v;  // ns <= e
+                        ++ns;
+                    } else if (b == bstar) {
+                        bnd[32 * nb + lane] = v;
+                        ++nb;
+                    } else {
+                        next = min(next, v);
+                    }
+                }
+                // the r smallest of the bucket (the words differ: each has its place
+                // in the stream), then the one after them
+                uint32_t last = 0u;
+                bool any = false;
+                KNN_LOOP_HINT
+                for (int i = 0; i <= r; ++i) {
+                    uint32_t best = i == r ? next : 0xffffffffu;
+                    KNN_LOOP_HINT
+                    for (int e = 0; e < nb; ++e) {
+                        const uint32_t v = bnd[32 * e + lane];
+                        if (!any || v > last) best = min(best, v);
+                    }
+                    if (i < r) {
+                        S.list[32 * (below + i) + lane] = best;
+                        last = best;
+                        any = true;
+                    } else {
+                        next = best;
+                    }
+                }
+                // exact set: the k-th stays inside R by more than the error bound,
+                // and the next candidate is more than twice the bound beyond it
+                const float unit = R2 * (1.0f / 1048575.0f);
+                T = ((float)(last >> 12) + 0.5f) * unit;
+                const float N = next == 0xffffffffu ? R2 : ((float)(next >> 12) - 0.5f) * unit;
+                const float e2 = 1.01f * eg + 2e-7f * R;
+                const float dT = sqrtf(T) * 1.000001f, dN = sqrtf(fmaxf(N, 0.0f)) * 0.999999f;
+                if (dT + 2.0f * e2 > R)
+                    reason = 3;
+                else if (dN - dT > 2.0f * e2)
+                    reason = 0;
+            }
+        }
+    }
+    // ---- rows of the accepted queries: places in the stream to slots ---------------------
+    if (act && reason == 0) {
+        int32_t *row = a.ngb + qi * k;
+        auto slot_at = [&](int e) -> int32_t {
+            const uint32_t g = S.list[32 * e + lane] & 4095u;
+            int j = 0;
+#pragma unroll
+            for (int st = kGroupRuns / 2; st > 0; st >>= 1)
+                if (j + st < nrun && S.off[j + st] <= g) j += st;
+            return (int32_t)(S.pa[j] + (g - S.off[j]));
+        };
+        if ((k & 3) == 0 && ((uintptr_t)a.ngb & 15) == 0) {
+            KNN_LOOP_HINT
+            for (int e = 0; e < k; e += 4)
+                *reinterpret_cast<int4 *>(row + e) = make_int4(slot_at(e), slot_at(e + 1), slot_at(e + 2), slot_at(e + 3));
+        } else {
+            KNN_LOOP_HINT
+            for (int e = 0; e < k; ++e) row[e] = slot_at(e);
+        }
+    }
+    // ---- everything else goes to the warp path -----------------------------------
+    const bool push = valid && !(act && reason == 0);
+    if (push) {
+        float Rnew = R;
+        if (reason == 1) {
+            const float g = 1.25f * powf((float)k / (float)max(cnt, 1), 1.0f / DIM);
+            Rnew = R * fminf(fmaxf(g, 1.25f), 4.0f);
+        } else if (reason == 3) {
+            Rnew = fmaxf(R, sqrtf(T) + 4.0f * (1.01f * eg + 2e-7f * R)) * 1.0001f;
+        }
+        a.radius[qi] = Rnew;
+    }
+    const unsigned pm = __ballot_sync(0xffffffffu, push);
+    if (pm) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(a.qout_count, __popc(pm));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (push) a.qout[base + __popc(pm & ((1u << lane) - 1u))] = (int32_t)qi;
+    }
+    // statistics: streamed candidates per member query, retries and their reasons
+    if (a.stats) {
+        const int na = __popc(__ballot_sync(0xffffffffu, act));
+        const int n1 = __popc(__ballot_sync(0xffffffffu, reason == 1));
+        const int n3 = __popc(__ballot_sync(0xffffffffu, reason == 3));
+#ifdef MG_KNN_GROUP_DEBUG
+        // [10] warps not streamed, [11] runs, [12] streamed, [13] outliers, [14]
+        // listed, [15] full lists
+        const int ol = __popc(__ballot_sync(0xffffffffu, valid && !mine));
+        const int fl = __popc(__ballot_sync(0xffffffffu, full));
+        const int lc = warp_sum(cnt);
+        if (lane == 0) {
+            unsigned long long *st = (unsigned long long *)a.stats;
+            atomicAdd(st + 10, ok ? 0ull : 1ull);
+            atomicAdd(st + 11, (unsigned long long)nrun);
+            atomicAdd(st + 12, (unsigned long long)tot);
+            atomicAdd(st + 13, (unsigned long long)ol);
+            atomicAdd(st + 14, (unsigned long long)lc);
+            atomicAdd(st + 15, (unsigned long long)fl);
+        }
+#endif
+        if (lane == 0) {
+            if (na) atomicAdd((unsigned long long *)&a.stats[1], (unsigned long long)na * (unsigned long long)tot);
+            if (pm) atomicAdd((unsigned long long *)&a.stats[2], (unsigned long long)__popc(pm));
+            if (n1) atomicAdd((unsigned long long *)&a.stats[6], (unsigned long long)n1);
+            if (n3) atomicAdd((unsigned long long *)&a.stats[8], (unsigned long long)n3);
+        }
+    }
+}
+
+// ---- first pass over a query list, one thread per query over a block's candidates ---
+// Slice and Reconstruct return FP64 values built on the FP32 derivatives of a
+// query list, in which the order of a row shows at ~1e-8; query lists keep the
+// search that has produced their rows so far (see the passes above), and with
+// it every bit of those results.
 // The G queries of a block are consecutive (neighbours in Morton order).  The
 // block looks up the cells over the bounding box of its queries' first-radius
 // spheres and stages, once, every particle inside the box of some warp's
@@ -1756,21 +2318,18 @@ __global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_hsml(cons
 // than 2e beyond the k-th (no other particle can change places with it).
 // Every other query (too few in radius, a near tie, a crowded boundary
 // bucket, a block whose staging overflows, a radius far above the block's
-// smallest) goes to the work queue, and the warp passes finish it.  Only the
+// smallest) goes to the work queue, and the passes finish it.  Only the
 // rows' slots are written (the order inside a row is the staging order); h is
 // solved from them by k_hsml_solve_rows with the warp path's FP32 hi/lo
 // distances (cand_d2p).
-constexpr int kGroupBins = 32;
-constexpr int kGroupList = 96;        // listed candidates per query
-constexpr int kGroupBoundary = 8;     // entries of the k-th neighbour's bucket kept per query
-constexpr int kGroupUnroll = 4;       // particles per thread per staging round
-#ifndef MG_KNN_GROUP_OUTLIER
-#define MG_KNN_GROUP_OUTLIER 2.0f
-#endif
-constexpr float kGroupOutlier = MG_KNN_GROUP_OUTLIER;  // radius above this multiple of the block's smallest: warp path
+constexpr int kBlockBins = 32;
+constexpr int kBlockBoundary = 8;  // entries of the k-th neighbour's bucket kept per query
+constexpr int kBlockUnroll = 4;    // particles per thread per staging round
+constexpr int kBlockThreads = 128; // queries per block
+constexpr int kBlockStage = 2048;  // staged candidates per block
 
 template <int G, int C>
-struct GroupSmem {
+struct BlockSmem {
     static constexpr int kWarps = G / 32;
     static constexpr int kWords = C / 32;
     static constexpr int kCells = 512;  // local Morton space of an 8 x 8 x 8 cell box
@@ -1780,9 +2339,9 @@ struct GroupSmem {
     float qbox[kWarps][6];              // per warp: box of its member queries' spheres
     uint16_t list[kGroupList * G];      // entry e of thread t at list_at(e, t); the
                                         // selected neighbours end up in the first k
-    uint16_t bnd[kGroupBoundary * G];   // boundary-bucket staged indices
-    float bnd_d[kGroupBoundary * G];    // and their d~^2
-    uint8_t hist[kGroupBins * G];       // per-thread bucket counts
+    uint16_t bnd[kBlockBoundary * G];   // boundary-bucket staged indices
+    float bnd_d[kBlockBoundary * G];    // and their d~^2
+    uint8_t hist[kBlockBins * G];       // per-thread bucket counts
     uint32_t cell_a[kCells];            // first slot of each box cell
     uint32_t cell_off[kCells + 1];      // prefix offsets of the cells' particles
     float red[8][kWarps];               // block reductions
@@ -1820,24 +2379,10 @@ __device__ __forceinline__ float group_d2(float cx, float cy, float cz, float qx
     return d2;
 }
 
-// Optional phase cycle counters of the first pass (build with
-// -DMG_KNN_GROUP_PROF): stats[10..15] accumulate, over warps, the clock64()
-// cycles of set-up and cell lookups, staging, the candidate scan, selection,
-// row writes, and hand-over.
-#ifdef MG_KNN_GROUP_PROF
-#define GROUP_TICK(i) \
-    do {              \
-        __syncwarp(); \
-        gt[i] = clock64(); \
-    } while (0)
-#else
-#define GROUP_TICK(i)
-#endif
-
 template <int DIM, int G, int C>
-__global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
+__global__ __launch_bounds__(G) void k_knn_group_block(const __grid_constant__ KnnPassArgs a) {
     extern __shared__ __align__(16) unsigned char group_smem[];
-    using SM = GroupSmem<G, C>;
+    using SM = BlockSmem<G, C>;
     static_assert(G % 64 == 0 && SM::kCells % G == 0, "list_at and the cell split need G = 64 m, G | 512");
     constexpr int NW = SM::kWarps;
     SM &S = *reinterpret_cast<SM *>(group_smem);
@@ -1848,10 +2393,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
     const float side = (float)fr.side;
     const float half_side = 0.5f * side;
     const int k = a.k;
-#ifdef MG_KNN_GROUP_PROF
-    long long gt[7];
-#endif
-    GROUP_TICK(0);
 
     int32_t p = 0;
     float4 h0 = make_float4(0.f, 0.f, 0.f, 0.f), l0 = h0;
@@ -1967,16 +2508,12 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
     // corners, key quantisation, offset rounding)
     const float cmarg = 2e-6f * side + 1e-3f * cside;
     __syncthreads();  // the warps' boxes
-    GROUP_TICK(1);
     // reason: 0 accepted, 1 too few in radius, 3 k-th too close to R, 4 other
     int reason = 4;
     int cnt = 0;
     float T = 0.0f;
     bool served = false;
     int my_nst = 0;
-#ifdef MG_KNN_GROUP_DEBUG
-    long long dbg_words = 0, dbg_iter = 0;
-#endif
     const float R2 = R * R;
     // Warps still to serve, served gsz at a time from the lowest: a block
     // whose staging overflows is staged again as two halves (re-staging smaller
@@ -2062,11 +2599,11 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
         for (int w = 0; w < NW; ++w)
 #pragma unroll
             for (int i = 0; i < 6; ++i) qb[w][i] = (wsel >> w & 1u) ? S.qbox[w][i] : (i < 3 ? FLT_MAX : -FLT_MAX);
-        // rounds of G * kGroupUnroll particles; the slots and loads of the next
+        // rounds of G * kBlockUnroll particles; the slots and loads of the next
         // round are issued before this round's compaction and barrier
-        auto fetch = [&](int base, uint32_t(&sl)[kGroupUnroll], float4(&hv)[kGroupUnroll],
-                         float4(&lv)[kGroupUnroll]) {
-            const int g0 = base + tid * kGroupUnroll;
+        auto fetch = [&](int base, uint32_t(&sl)[kBlockUnroll], float4(&hv)[kBlockUnroll],
+                         float4(&lv)[kBlockUnroll]) {
+            const int g0 = base + tid * kBlockUnroll;
             int c = 0;
             if (g0 < tot) {
                 int hi_c = ncell;
@@ -2079,7 +2616,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kGroupUnroll; ++u) {
+            for (int u = 0; u < kBlockUnroll; ++u) {
                 const int g = g0 + u;
                 sl[u] = 0xffffffffu;
                 if (g < tot) {
@@ -2088,7 +2625,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kGroupUnroll; ++u) {
+            for (int u = 0; u < kBlockUnroll; ++u) {
                 if (sl[u] != 0xffffffffu) {
                     hv[u] = a.hi[sl[u]];
                     lv[u] = a.lo[sl[u]];
@@ -2098,19 +2635,19 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
             }
         };
-        uint32_t slot[kGroupUnroll];
-        float4 hb[kGroupUnroll], lb[kGroupUnroll];
+        uint32_t slot[kBlockUnroll];
+        float4 hb[kBlockUnroll], lb[kBlockUnroll];
         if (tot > 0) fetch(0, slot, hb, lb);
         int round = 0;
-        for (int base = 0; base < tot; base += G * kGroupUnroll, ++round) {
-            uint32_t slot_n[kGroupUnroll];
-            float4 hb_n[kGroupUnroll], lb_n[kGroupUnroll];
-            if (base + G * kGroupUnroll < tot) fetch(base + G * kGroupUnroll, slot_n, hb_n, lb_n);
-            float ox_[kGroupUnroll], oy_[kGroupUnroll], oz_[kGroupUnroll];
+        for (int base = 0; base < tot; base += G * kBlockUnroll, ++round) {
+            uint32_t slot_n[kBlockUnroll];
+            float4 hb_n[kBlockUnroll], lb_n[kBlockUnroll];
+            if (base + G * kBlockUnroll < tot) fetch(base + G * kBlockUnroll, slot_n, hb_n, lb_n);
+            float ox_[kBlockUnroll], oy_[kBlockUnroll], oz_[kBlockUnroll];
             int nkeep = 0;
             unsigned keepm = 0;
 #pragma unroll
-            for (int u = 0; u < kGroupUnroll; ++u) {
+            for (int u = 0; u < kBlockUnroll; ++u) {
                 float ox = 0.0f, oy = 0.0f, oz = 0.0f;
                 if (DIM > 0) ox = __fadd_rn(__fsub_rn(hb[u].x, ctr[0]), lb[u].x);
                 if (DIM > 1) oy = __fadd_rn(__fsub_rn(hb[u].y, ctr[1]), lb[u].y);
@@ -2142,7 +2679,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             }
             int pos = nst + woff + inc - nkeep;
 #pragma unroll
-            for (int u = 0; u < kGroupUnroll; ++u) {
+            for (int u = 0; u < kBlockUnroll; ++u) {
                 if (keepm >> u & 1u) {
                     if (pos < C) {
                         S.sx[pos] = ox_[u];
@@ -2155,7 +2692,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             }
             nst += btot;
 #pragma unroll
-            for (int u = 0; u < kGroupUnroll; ++u) {
+            for (int u = 0; u < kBlockUnroll; ++u) {
                 slot[u] = slot_n[u];
                 hb[u] = hb_n[u];
                 lb[u] = lb_n[u];
@@ -2195,7 +2732,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
     }
     __syncthreads();
 
-    GROUP_TICK(2);
     // ---- per-thread selection ----------------------------------------------------
     const bool act = stage_ok && mine && (wsel >> wib & 1u);
     if (act) {
@@ -2231,9 +2767,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
                 if (!__any_sync(0xffffffffu, bd2 <= R2w)) continue;
             }
-#ifdef MG_KNN_GROUP_DEBUG
-            ++dbg_words;
-#endif
             // the word's 32 distances first (independent loads, two per packed
             // instruction), then the list; bit b set when R^2 - d~^2 >= 0
             uint32_t mp[4] = {0u, 0u, 0u, 0u};
@@ -2265,9 +2798,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
             }
             uint32_t m = (mp[0] | mp[1]) | (mp[2] | mp[3]);
-#ifdef MG_KNN_GROUP_DEBUG
-            dbg_iter += __reduce_max_sync(0xffffffffu, (unsigned)__popc(m));
-#endif
             while (m) {
                 const int b = __ffs(m) - 1;
                 m &= m - 1;
@@ -2276,7 +2806,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             }
         }
     }
-    GROUP_TICK(3);
     if (act) {
         if (cnt < k) {
             reason = 1;
@@ -2284,7 +2813,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             // B: histogram of the list in 32 buckets of d~^2 / R^2
             const float bscale = 32.0f / R2;
 #pragma unroll
-            for (int b = 0; b < kGroupBins; ++b) S.hist[hist_at<G>(b, tid)] = 0;
+            for (int b = 0; b < kBlockBins; ++b) S.hist[hist_at<G>(b, tid)] = 0;
             KNN_LOOP_HINT
             for (int e0 = 0; e0 < cnt; e0 += 4) {
                 int bk[4];
@@ -2293,15 +2822,15 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                     const int e = min(e0 + u, cnt - 1);
                     const int j = S.list[list_at(e, tid)];
                     const float d2 = group_d2<DIM>(S.sx[j], S.sy[j], S.sz[j], qx, qy, qz);
-                    bk[u] = e0 + u < cnt ? min(kGroupBins - 1, (int)(d2 * bscale)) : -1;
+                    bk[u] = e0 + u < cnt ? min(kBlockBins - 1, (int)(d2 * bscale)) : -1;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (bk[u] >= 0) ++S.hist[hist_at<G>(bk[u], tid)];
             }
-            int cum = 0, bstar = kGroupBins - 1, c_lo = 0, m_b = 0;
+            int cum = 0, bstar = kBlockBins - 1, c_lo = 0, m_b = 0;
             KNN_LOOP_HINT
-            for (int b = 0; b < kGroupBins; ++b) {
+            for (int b = 0; b < kBlockBins; ++b) {
                 const int h = S.hist[hist_at<G>(b, tid)];
                 if (cum + h >= k) {
                     bstar = b;
@@ -2311,7 +2840,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                 }
                 cum += h;
             }
-            if (m_b <= kGroupBoundary) {
+            if (m_b <= kBlockBoundary) {
                 // C: buckets below taken whole, the boundary bucket kept aside
                 int nsure = 0, nb = 0;
                 float nextmin = R2;  // anything not listed lies beyond R
@@ -2324,7 +2853,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                         const int e = min(e0 + u, cnt - 1);
                         jj[u] = S.list[list_at(e, tid)];
                         dd[u] = group_d2<DIM>(S.sx[jj[u]], S.sy[jj[u]], S.sz[jj[u]], qx, qy, qz);
-                        bk[u] = e0 + u < cnt ? min(kGroupBins - 1, (int)(dd[u] * bscale)) : kGroupBins;
+                        bk[u] = e0 + u < cnt ? min(kBlockBins - 1, (int)(dd[u] * bscale)) : kBlockBins;
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
@@ -2337,7 +2866,7 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
                                 S.bnd_d[nb * G + tid] = dd[u];
                             }
                             ++nb;
-                        } else if (bk[u] < kGroupBins) {
+                        } else if (bk[u] < kBlockBins) {
                             nextmin = fminf(nextmin, dd[u]);
                         }
                     }
@@ -2386,7 +2915,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
         }
     }
 
-    GROUP_TICK(4);
     // ---- rows of the accepted queries (coalesced, one row per warp step) ---------
     const unsigned acc = __ballot_sync(0xffffffffu, act && reason == 0);
     if (acc) {
@@ -2405,7 +2933,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
     todo &= ~wsel;
     __syncthreads();  // the next group restages the shared buffers
     }
-    GROUP_TICK(5);
     // ---- everything else goes to the warp passes -----------------------------------
     const bool push = valid && !(served && reason == 0);
     if (push) {
@@ -2417,6 +2944,8 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
             Rnew = fmaxf(R, sqrtf(T) + 4.0f * (1.01f * eg + 2e-7f * R)) * 1.0001f;
         }
         a.radius[qi] = Rnew;
+        a.rlo[qi] = 0.0f;
+        a.rhi[qi] = 0.0f;
     }
     const unsigned pm = __ballot_sync(0xffffffffu, push);
     if (pm) {
@@ -2425,32 +2954,6 @@ __global__ __launch_bounds__(G) void k_knn_group(KnnArgs a) {
         base = __shfl_sync(0xffffffffu, base, 0);
         if (push) a.qout[base + __popc(pm & ((1u << lane) - 1u))] = (int32_t)qi;
     }
-#ifdef MG_KNN_GROUP_PROF
-    GROUP_TICK(6);
-    if (lane == 0 && a.stats)
-        for (int i = 0; i < 6; ++i) atomicAdd((unsigned long long *)&a.stats[10 + i], (unsigned long long)(gt[i + 1] - gt[i]));
-#endif
-#ifdef MG_KNN_GROUP_DEBUG
-    // [10] blocks whose staging failed, [11] words scanned summed over warps,
-    // [12] member queries pushed for another reason, [13] outliers, [14]
-    // listed candidates summed over members, [15] list-append iterations
-    // summed over warps
-    if (a.stats) {
-        const int r4 = __popc(__ballot_sync(0xffffffffu, served && reason == 4));
-        const int ol = __popc(__ballot_sync(0xffffffffu, valid && !mine));
-        const int64_t lc = warp_sum<int64_t>(served ? (int64_t)cnt : 0);
-        if (tid == 0 && !geom_ok) atomicAdd((unsigned long long *)&a.stats[10], 1ull);
-        if (lane == 0) {
-            atomicAdd((unsigned long long *)&a.stats[11], (unsigned long long)dbg_words);
-            atomicAdd((unsigned long long *)&a.stats[15], (unsigned long long)dbg_iter);
-        }
-        if (lane == 0) {
-            if (r4) atomicAdd((unsigned long long *)&a.stats[12], (unsigned long long)r4);
-            if (ol) atomicAdd((unsigned long long *)&a.stats[13], (unsigned long long)ol);
-            if (lc) atomicAdd((unsigned long long *)&a.stats[14], (unsigned long long)lc);
-        }
-    }
-#endif
     // statistics: staged candidates per member query, retries and their reasons
     if (a.stats) {
         const int64_t cand = warp_sum<int64_t>(served ? (int64_t)my_nst : 0);
@@ -2991,33 +3494,41 @@ static int launch_pass_t(unsigned blocks, unsigned heavy_blocks, cudaStream_t st
 
 template <int DIM>
 static int launch_pass_d(int k, unsigned blocks, unsigned heavy_blocks, cudaStream_t st, const KnnPassArgs &a) {
+    if (k <= 32) return launch_pass_t<DIM, 1>(blocks, heavy_blocks, st, a);
     return k <= 64 ? launch_pass_t<DIM, 2>(blocks, heavy_blocks, st, a)
                    : launch_pass_t<DIM, 4>(blocks, heavy_blocks, st, a);
 }
 
-#ifndef MG_KNN_GROUP_G
-#define MG_KNN_GROUP_G 128
-#endif
-#ifndef MG_KNN_GROUP_C
-#define MG_KNN_GROUP_C 2048
-#endif
-constexpr int kGroupThreads = MG_KNN_GROUP_G;  // queries per block of the first pass
-constexpr int kGroupStage = MG_KNN_GROUP_C;    // staged candidates per block
-
 template <int DIM>
-static int launch_group_d(unsigned blocks, cudaStream_t st, const KnnArgs &a) {
-    const size_t smem = sizeof(GroupSmem<kGroupThreads, kGroupStage>);
-    MG_CUDA(cudaFuncSetAttribute(k_knn_group<DIM, kGroupThreads, kGroupStage>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_knn_group<DIM, kGroupThreads, kGroupStage><<<blocks, kGroupThreads, smem, st>>>(a);
+static int launch_group_d(cudaStream_t st, const KnnArgs &a) {
+    auto fn = a.periodic ? k_knn_group<DIM, true> : k_knn_group<DIM, false>;
+    const size_t smem = sizeof(GroupSmem) * kGroupWarps;
+    MG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fn<<<(unsigned)((a.nq + 32 * kGroupWarps - 1) / (32 * kGroupWarps)), 32 * kGroupWarps, smem, st>>>(a);
     MG_CHECK_LAUNCH();
     return MG_OK;
 }
 
-static int launch_group(int dim, unsigned blocks, cudaStream_t st, const KnnArgs &a) {
-    if (dim == 1) return launch_group_d<1>(blocks, st, a);
-    if (dim == 2) return launch_group_d<2>(blocks, st, a);
-    return launch_group_d<3>(blocks, st, a);
+static int launch_group(int dim, cudaStream_t st, const KnnArgs &a) {
+    if (dim == 1) return launch_group_d<1>(st, a);
+    if (dim == 2) return launch_group_d<2>(st, a);
+    return launch_group_d<3>(st, a);
+}
+
+template <int DIM>
+static int launch_group_block_d(cudaStream_t st, const KnnPassArgs &a) {
+    auto fn = k_knn_group_block<DIM, kBlockThreads, kBlockStage>;
+    const size_t smem = sizeof(BlockSmem<kBlockThreads, kBlockStage>);
+    MG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fn<<<(unsigned)((a.nq + kBlockThreads - 1) / kBlockThreads), kBlockThreads, smem, st>>>(a);
+    MG_CHECK_LAUNCH();
+    return MG_OK;
+}
+
+static int launch_group_block(int dim, cudaStream_t st, const KnnPassArgs &a) {
+    if (dim == 1) return launch_group_block_d<1>(st, a);
+    if (dim == 2) return launch_group_block_d<2>(st, a);
+    return launch_group_block_d<3>(st, a);
 }
 
 // process-wide switch of the first (group) pass; atomic so that a call on
@@ -3082,17 +3593,16 @@ extern "C" size_t mg_knn_hsml_workspace_bytes(int64_t nq, int32_t k) {
     if (nq <= 0 || k < 1) return 0;
     // the selected-distance rows are scratch of the h solve only for k > 32
     const size_t dsel_entries = k > 32 ? (size_t)nq * (size_t)k : 0;
-    size_t b = align_up(sizeof(float) * nq) + align_up(sizeof(int32_t) * nq) + align_up(sizeof(int32_t) * 64) + 1024;
-    if (k > 32)  // brackets, second queue, heavy items and their counters
-        b += align_up(sizeof(float) * dsel_entries) + 2 * align_up(sizeof(float) * nq) +
-             align_up(sizeof(int32_t) * nq) + align_up(sizeof(int32_t) * (size_t)heavy_capacity(nq) * kHeavyItem) +
-             2 * align_up(sizeof(int32_t) * 64);
-    return b;
+    return 3 * align_up(sizeof(float) * nq) + 2 * align_up(sizeof(int32_t) * nq) +
+           align_up(sizeof(float) * dsel_entries) +
+           align_up(sizeof(int32_t) * (size_t)heavy_capacity(nq) * kHeavyItem) + 3 * align_up(sizeof(int32_t) * 64) +
+           1024;
 }
 
-// The search of k > 32: max_passes passes over the queue.
-static int knn_passes(const mg_cells *c, const KnnArgs &a0, int max_passes, int nsm, int32_t *counts, Carve &w,
-                      cudaStream_t st) {
+// The search of k > 32 and of query lists: max_passes passes over the queue, the
+// first one thread per query where it may be (block_first).
+static int knn_passes(const mg_cells *c, const KnnArgs &a0, bool block_first, int max_passes, int nsm,
+                      int32_t *counts, Carve &w, cudaStream_t st) {
     KnnPassArgs a;
     static_cast<KnnArgs &>(a) = a0;
     const int64_t nq = a.nq, hcap = heavy_capacity(nq);
@@ -3120,6 +3630,11 @@ static int knn_passes(const mg_cells *c, const KnnArgs &a0, int max_passes, int 
         if (pass > 0) {
             k_count_pass<<<1, 32, 0, st>>>(counts + (pass - 1), a.stats);
             MG_CHECK_LAUNCH();
+        }
+        if (pass == 0 && block_first) {
+            const int rc = launch_group_block(c->dim, st, a);
+            if (rc) return rc;
+            continue;
         }
         const int rc = launch_pass(c->dim, (unsigned)std::min<int64_t>(blocks, 2147483647), (unsigned)nsm * 4, st, a);
         if (rc) return rc;
@@ -3171,19 +3686,19 @@ extern "C" int mg_knn_hsml(const mg_cells *c, const int32_t *queries, int64_t nq
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // first pass one thread per query over block-shared candidates (not for
-    // periodic boxes or k > 32; its leftovers go to the warp path)
-    const bool group_first = g_group_pass.load() && !a.periodic && k <= 32 && max_passes >= 2;
-    if (group_first) {
-        const int rc = launch_group(c->dim, (unsigned)((nq + kGroupThreads - 1) / kGroupThreads), st, a);
-        if (rc) return rc;
-        a.qin = queue;
-        a.qin_count = counts;
-    }
-    if (k > 32) {
-        const int rc = knn_passes(c, a, max_passes, nsm, counts, w, st);
+    const bool group = g_group_pass.load() && k <= 32 && max_passes >= 2;
+    if (k > 32 || queries) {
+        const int rc = knn_passes(c, a, group && !a.periodic, max_passes, nsm, counts, w, st);
         if (rc) return rc;
     } else {
+        // first pass one thread per query over its warp's candidates; its leftovers
+        // go to the warp path
+        if (group) {
+            const int rc = launch_group(c->dim, st, a);
+            if (rc) return rc;
+            a.qin = queue;
+            a.qin_count = counts;
+        }
         // persistent warps, as many blocks as the SMs hold at once
         const int64_t blocks = std::min((int64_t)nsm * kKnnMinBlocks, (nq + kKnnWarps - 1) / kKnnWarps);
         const int rc = launch_knn(c->dim, (unsigned)blocks, st, a);
