@@ -16,6 +16,7 @@
 #include <cfloat>
 
 #include "mg_common.cuh"
+#include "mg_f32x2.cuh"
 #include "mg_maps.cuh"
 #include "mg_scan.cuh"
 
@@ -30,6 +31,14 @@ struct SdParticle {
     float coef;     // f / h^2 (standard) or f / total_weight (conservative)
     int gx0, gx1, gy0, gy1;
 };
+
+// Pairs per work item of k_sd_tile: as many as give some 16 items per SM, within
+// these limits (a large item amortises its tile's set-up and store; 65,536
+// uniform points on a 256^2 map fill 128 items of 2048, fewer than there are
+// SMs, and took 0.40 ms).
+constexpr int kSdChunk = 2048, kSdChunkMin = 256, kSdItemsPerSm = 16;
+constexpr int kSdBigChunk = 1024;  // pairs per work item of k_sd_tile_pairs
+constexpr int kSdWarps = 8;        // warps per block of k_sd_tile, each with its own copy of the tile
 
 struct SdArgs {
     const double *pos;
@@ -52,10 +61,13 @@ struct SdArgs {
     int32_t *bpairs;      // bcap: particle of each pair, grouped by tile
     uint32_t *bitem_off;  // ntiles + 1: first work item of each tile (chunks of kSdBigChunk pairs)
     uint64_t bcap;
+    int nsm;
 };
 
-constexpr int kSdChunk = 2048;     // pairs per work item of k_sd_tile
-constexpr int kSdBigChunk = 1024;  // pairs per work item of k_sd_tile_pairs
+__host__ __device__ inline uint32_t sd_chunk(uint64_t pairs, int nsm) {
+    const uint64_t c = pairs / (uint64_t)(kSdItemsPerSm * nsm);
+    return (uint32_t)(c < kSdChunkMin ? kSdChunkMin : (c > kSdChunk ? kSdChunk : c));
+}
 
 // Footprint of particle i exactly as the reference computes it (FP64, C
 // truncation toward zero), grid_deposition.py:200-216 / :248-265.
@@ -265,23 +277,31 @@ __global__ void k_sd_scatter(SdArgs a) {
     }
 }
 
-// Work items per tile: ceil(pairs / kSdChunk), at least 1 (an empty tile still
+// Work items per tile: ceil(pairs / chunk), at least 1 (an empty tile still
 // writes its zeros).
 __global__ void k_sd_items(SdArgs a, int64_t ntiles) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t < ntiles) {
         const uint32_t c = a.tile_count[t + 1] - a.tile_count[t];
-        a.item_off[t] = c <= (uint32_t)kSdChunk ? 1u : (c + kSdChunk - 1) / kSdChunk;
+        const uint32_t chunk = sd_chunk(a.tile_count[ntiles], a.nsm);
+        a.item_off[t] = c <= chunk ? 1u : (c + chunk - 1) / chunk;
     } else if (t == ntiles) {
         a.item_off[t] = 0u;
     }
 }
 
-// One CTA per work item (a tile, or a chunk of kSdChunk pairs of a crowded
-// tile): shared-memory accumulation; a tile of one item stores its pixels, the
-// chunks of a split tile add theirs atomically into the zeroed grid.
-__global__ __launch_bounds__(256) void k_sd_tile(SdArgs a, int64_t ntiles) {
-    __shared__ float acc[kTile][kTile + 1];
+// One CTA per work item (a tile, or a chunk of a crowded tile's pairs).  A warp
+// takes one pair at a time, its lanes over the footprint's pixels, and adds to
+// its own copy of the tile in shared memory by plain reads and writes: the lanes
+// of a pair hit different pixels, so that no atomic is needed (a float add to
+// shared memory is a compare-and-swap loop).  The copies are summed at the end; a
+// tile of one item stores its pixels, the chunks of a split tile add theirs
+// atomically into the zeroed grid.  The next pair's record is loaded while this
+// one is added.  Bound: instruction issue (~25 per 32 pixels).  2^20 Plummer
+// particles, 1024^2 pixels: 1.02 -> 0.74 ms; 65,536 uniform points, 256^2 pixels
+// (with the smaller items): 0.40 -> 0.08 ms.
+__global__ __launch_bounds__(32 * kSdWarps) void k_sd_tile(SdArgs a, int64_t ntiles) {
+    __shared__ float acc[kSdWarps][kTile * (kTile + 1)];
     const uint32_t item = blockIdx.x;
     if (item >= a.item_off[ntiles]) return;
     int64_t lo = 0, hi = ntiles - 1;  // tile: largest t with item_off[t] <= item
@@ -296,15 +316,22 @@ __global__ __launch_bounds__(256) void k_sd_tile(SdArgs a, int64_t ntiles) {
     const uint32_t nitems = a.item_off[tile + 1] - a.item_off[tile];
     const uint32_t j = item - a.item_off[tile];
     const int tx = tile / a.ntx, ty = tile % a.ntx;
-    for (int e = threadIdx.x; e < kTile * kTile; e += blockDim.x) acc[e / kTile][e % kTile] = 0.0f;
-    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *own = acc[warp];
+    for (int e = lane; e < kTile * (kTile + 1); e += 32) own[e] = 0.0f;
+    __syncwarp();
+    const uint32_t chunk = sd_chunk(a.tile_count[ntiles], a.nsm);
     const uint32_t t0 = a.tile_count[tile], t1 = a.tile_count[tile + 1];
-    const uint32_t b0 = t0 + j * (uint32_t)kSdChunk, b1 = min(t1, b0 + (uint32_t)kSdChunk);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const uint32_t b0 = t0 + j * chunk, b1 = min(t1, b0 + chunk);
     const float dxf = (float)a.dx;
     const int px0 = tx * kTile, py0 = ty * kTile;
-    for (uint32_t e = b0 + warp; e < b1; e += nwarp) {
-        const SdParticle r = a.rec[a.pairs[e]];
+    SdParticle next;
+    next.gx0 = 0;
+    next.gx1 = -1;
+    if (b0 + warp < b1) next = a.rec[a.pairs[b0 + warp]];
+    for (uint32_t e = b0 + warp; e < b1; e += kSdWarps) {
+        const SdParticle r = next;
+        if (e + kSdWarps < b1) next = a.rec[a.pairs[e + kSdWarps]];
         const int x0 = max(r.gx0, px0), x1 = min(r.gx1, px0 + kTile - 1);
         const int y0 = max(r.gy0, py0), y1 = min(r.gy1, py0 + kTile - 1);
         const int w = x1 - x0 + 1, hgt = y1 - y0 + 1;
@@ -317,7 +344,7 @@ __global__ __launch_bounds__(256) void k_sd_tile(SdArgs a, int64_t ntiles) {
         // footprint's first node as exact small floats; |d| by r^2 rsqrt(r^2)
         const float h2 = r.h * r.h, hf = (float)hgt, inv = 1.0f / hf;
         const float fx0 = (float)(x0 - r.gx0), fy0 = (float)(y0 - r.gy0);
-        float *accf = &acc[0][0] + (x0 - px0) * (kTile + 1) + (y0 - py0);
+        float *accf = own + (x0 - px0) * (kTile + 1) + (y0 - py0);
         const int skew = kTile + 1 - hgt;
         for (int t = lane; t < w * hgt; t += 32) {
             const float tf = (float)t;
@@ -327,15 +354,19 @@ __global__ __launch_bounds__(256) void k_sd_tile(SdArgs a, int64_t ntiles) {
             const float ddy = fmaf(-(fy0 + cf), dxf, r.ry);
             const float r2 = fmaf(ddx, ddx, ddy * ddy);
             if (r2 > h2) continue;
-            atomicAdd(accf + t + (int)rf * skew, spline_w_half(r2 * rsqrtf(fmaxf(r2, 1e-30f)) * hinv) * coef2);
+            accf[t + (int)rf * skew] += spline_w_half(r2 * rsqrtf(fmaxf(r2, 1e-30f)) * hinv) * coef2;
         }
+        __syncwarp();  // the next pair's lanes read what these wrote
     }
     __syncthreads();
     const double scale = a.conservative ? 1.0 / (a.dx * a.dx) : 1.0;
     for (int e = threadIdx.x; e < kTile * kTile; e += blockDim.x) {
         const int gx = px0 + e / kTile, gy = py0 + e % kTile;
         if (gx >= a.res || gy >= a.res) continue;
-        const double v = (double)acc[e / kTile][e % kTile] * scale;
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSdWarps; ++k) v += (double)acc[k][(e / kTile) * (kTile + 1) + e % kTile];
+        v *= scale;
         if (nitems == 1)
             a.grid[(int64_t)gx * a.res + gy] = v;
         else if (v != 0.0)
@@ -510,7 +541,9 @@ __global__ void k_sd_big_items(SdArgs a, int64_t ntiles) {
 // holds every node within h of the particle along each axis (the
 // truncations of footprint()), so a node outside it lies at q >= 1 and
 // weighs exactly 0, up to the FP32 rounding of q near 1 (a weight below
-// 1e-18 of the peak; tests/native/sd_cull_check.cu).  A tile of one item adds its values to the pixels
+// 1e-18 of the peak; tests/native/sd_cull_check.cu).  The pixels go two to a
+// packed instruction (each half rounds as before: the same bits): 2^20 Plummer
+// particles, 1024^2 pixels 1.50 -> 1.43 ms, bound by the FP32 pipe.  A tile of one item adds its values to the pixels
 // k_sd_tile wrote; the items of a split tile add theirs with FP64 atomics.
 __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles) {
     __shared__ float4 sa[256];  // rx, ry, 1/h, 2 coef * norm
@@ -519,6 +552,8 @@ __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles)
     const uint32_t nitems = a.bitem_off[ntiles];
     const int tid = threadIdx.x;
     const float dxf = (float)a.dx;
+    const unsigned long long mdx = f2_pack(-dxf), three = f2_pack(3.0f), mthree = f2_pack(-3.0f),
+                             half = f2_pack(0.5f), one = f2_pack(1.0f);
     const double scale = a.conservative ? 1.0 / (a.dx * a.dx) : 1.0;
     for (uint32_t item = blockIdx.x; item < nitems; item += gridDim.x) {
         int64_t lo = 0, hi = ntiles - 1;  // tile: largest t with bitem_off[t] <= item
@@ -536,12 +571,11 @@ __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles)
         const int bx0 = tx * kTile + 16 * ((tid >> 5) & 1), by0 = ty * kTile + 8 * (tid >> 6);  // the warp's sub-block
         const int gy = by0 + (tid & 7), gxb = bx0 + ((tid >> 3) & 3);
         const float fgy = (float)gy, fbx0 = (float)bx0, fby0 = (float)by0;
-        float fgx[4];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) fgx[jj] = (float)(gxb + 4 * jj);
+        const unsigned long long fgx[2] = {f2_pack((float)gxb, (float)(gxb + 4)),
+                                           f2_pack((float)(gxb + 8), (float)(gxb + 12))};
         const uint32_t p0 = a.btile[tile] + j * (uint32_t)kSdBigChunk;
         const uint32_t p1 = min(a.btile[tile + 1], p0 + (uint32_t)kSdBigChunk);
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        unsigned long long acc2[2] = {0ull, 0ull};
         for (uint32_t c0 = p0; c0 < p1; c0 += 256) {
             __syncthreads();  // the previous batch is consumed
             if (c0 + tid < p1) {
@@ -556,16 +590,28 @@ __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles)
                 if (sd_block_skips(fbx0, fby0, pa, pb, dxf)) continue;  // warp-uniform
                 const float oy = fgy - pb.z;  // exact: gy - gy0
                 const float ddy = fmaf(-oy, dxf, pa.y);
-                const float ddy2 = ddy * ddy;
+                const unsigned long long ddy2 = f2_pack(ddy * ddy), rx = f2_pack(pa.x), hinv = f2_pack(pa.z),
+                                         coef = f2_pack(pa.w), gx0 = f2_pack(pb.x);
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const float ox = fgx[jj] - pb.x;  // exact: gx - gx0
-                    const float ddx = fmaf(-ox, dxf, pa.x);
-                    const float r2 = fmaf(ddx, ddx, ddy2);
-                    acc[jj] = fmaf(spline_w_half(r2 * rsqrtf(fmaxf(r2, 1e-30f)) * pa.z), pa.w, acc[jj]);
+                for (int u = 0; u < 2; ++u) {
+                    const unsigned long long ox = f2_sub(fgx[u], gx0);  // exact: gx - gx0
+                    const unsigned long long ddx = f2_fma(ox, mdx, rx);
+                    const unsigned long long r2 = f2_fma(ddx, ddx, ddy2);
+                    const unsigned long long rs = f2_pack(rsqrtf(fmaxf(f2_low(r2), 1e-30f)),
+                                                          rsqrtf(fmaxf(f2_high(r2), 1e-30f)));
+                    const unsigned long long q = f2_mul(f2_mul(r2, rs), hinv);
+                    // spline_w_half of both
+                    const unsigned long long in = f2_fma(f2_mul(q, q), f2_fma(three, q, mthree), half);
+                    const unsigned long long c = f2_sub(one, q);
+                    const unsigned long long am = f2_pack(fmaxf(f2_low(c), 0.0f), fmaxf(f2_high(c), 0.0f));
+                    const unsigned long long out = f2_mul(f2_mul(am, am), am);
+                    const unsigned long long w = f2_pack(f2_low(q) <= 0.5f ? f2_low(in) : f2_low(out),
+                                                         f2_high(q) <= 0.5f ? f2_high(in) : f2_high(out));
+                    acc2[u] = f2_fma(w, coef, acc2[u]);
                 }
             }
         }
+        const float acc[4] = {f2_low(acc2[0]), f2_high(acc2[0]), f2_low(acc2[1]), f2_high(acc2[1])};
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
             const int gx = gxb + 4 * jj;
@@ -931,6 +977,11 @@ extern "C" int mg_surface_density(const double *pos, const double *h, const doub
     a.bfill = w.take<uint32_t>(ntiles + 1);
     a.bitem_off = w.take<uint32_t>(ntiles + 1);
     a.bcap = sd_big_capacity(n);
+    int dev = 0;
+    a.nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&a.nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nsm = a.nsm;
     a.bpairs = w.take<int32_t>(a.bcap);
     if (!w.ok()) return MG_ERR_ARG;
     MG_CUDA(cudaMemsetAsync(a.tile_count, 0, sizeof(uint32_t) * (ntiles + 1), st));
@@ -940,9 +991,6 @@ extern "C" int mg_surface_density(const double *pos, const double *h, const doub
     const unsigned nb = (unsigned)((n + 255) / 256);
     k_sd_prep<<<nb, 256, 0, st>>>(a);
     MG_CHECK_LAUNCH();
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (conservative) {
         k_sd_cons_norm<<<(unsigned)(nsm * 8), 256, 0, st>>>(a);
         MG_CHECK_LAUNCH();
@@ -958,8 +1006,11 @@ extern "C" int mg_surface_density(const double *pos, const double *h, const doub
     MG_CHECK_LAUNCH();
     rc = exclusive_scan_u32(a.item_off, a.item_off, ntiles + 1, scan_ws, st);
     if (rc) return rc;
-    const int64_t max_items = ntiles + (4 * n) / kSdChunk + 1;
-    k_sd_tile<<<(unsigned)max_items, 256, 0, st>>>(a, ntiles);
+    // (pairs / chunk: at most kSdItemsPerSm per SM and one, unless the chunk is at a limit)
+    const int64_t max_items = ntiles + 1 + std::max<int64_t>((4 * n) / kSdChunk,
+                                                             std::min<int64_t>((4 * n) / kSdChunkMin,
+                                                                               (int64_t)(kSdItemsPerSm + 1) * nsm));
+    k_sd_tile<<<(unsigned)max_items, 32 * kSdWarps, 0, st>>>(a, ntiles);
     MG_CHECK_LAUNCH();
     // large footprints: per-tile pairs when they fit the buffer (decided on
     // the device from the count), else the gather or the FP64-atomic path
