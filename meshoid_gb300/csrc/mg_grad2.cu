@@ -30,10 +30,9 @@
 
 namespace mg {
 
-constexpr int kG2NF = 4;       // components per rhs launch
 constexpr int kG2FixG = 4;     // components per right-hand-side pass of the FP64 re-solve
 #ifndef MG_G2_RHS_MINB
-#define MG_G2_RHS_MINB 2  // resident blocks of k_g2_rhs per SM the registers are cut for
+#define MG_G2_RHS_MINB 4  // resident blocks of k_g2_rhs per SM the registers are cut for
 #endif
 
 struct G2Args {
@@ -125,8 +124,27 @@ __global__ __launch_bounds__(128) void k_g2_moments(const __grid_constant__ G2Ar
     if (flag) g.queue[atomicAdd(g.qcount, 1)] = (int32_t)q;
 }
 
+// NF consecutive floats at p, aligned to their size (a row holds a multiple of 4).
+template <int NF>
+__device__ __forceinline__ void g2_load(const float *__restrict__ p, float v[NF]) {
+    if constexpr (NF == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (NF == 2) {
+        const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        v[0] = __ldg(p);
+    }
+}
+
+// Right-hand sides and solutions of NF = 1, 2 or 4 components: as many as there
+// are left, not padded to 4, whose float-float sums (nine per component and
+// neighbour) are most of the work.  131,071 Plummer particles, k = 64, 2
+// components: 0.41 -> 0.21 ms a call (half the sums, and registers for four
+// blocks per SM instead of two; three or five: 0.30, 0.21 ms).
 template <int DIM, int NF>
-__global__ __launch_bounds__(128, MG_G2_RHS_MINB) void k_g2_rhs(const __grid_constant__ G2Args g) {
+__global__ __launch_bounds__(128, NF == 4 ? 2 : MG_G2_RHS_MINB) void k_g2_rhs(const __grid_constant__ G2Args g) {
     constexpr int ND = G2<DIM>::ND, NM = G2<DIM>::NM;
     __shared__ float2 sb[NF * ND * 128];  // [component * ND + m][thread]: normalised right-hand sides
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < g.nq;
@@ -138,15 +156,9 @@ __global__ __launch_bounds__(128, MG_G2_RHS_MINB) void k_g2_rhs(const __grid_con
         const ff hinv = g2_hinv(g, q);
         float f0h[NF], f0m[NF], f0l[NF];
         const int64_t r0 = (int64_t)p * g.nfp + g.c0;
-#pragma unroll
-        for (int c = 0; c < NF; c += 4) {
-            const float4 vh = *reinterpret_cast<const float4 *>(g.f_hi + r0 + c);
-            const float4 vm = *reinterpret_cast<const float4 *>(g.f_mid + r0 + c);
-            const float4 vl = *reinterpret_cast<const float4 *>(g.f_lo + r0 + c);
-            f0h[c] = vh.x; f0h[c + 1] = vh.y; f0h[c + 2] = vh.z; f0h[c + 3] = vh.w;
-            f0m[c] = vm.x; f0m[c + 1] = vm.y; f0m[c + 2] = vm.z; f0m[c + 3] = vm.w;
-            f0l[c] = vl.x; f0l[c + 1] = vl.y; f0l[c + 2] = vl.z; f0l[c + 3] = vl.w;
-        }
+        g2_load<NF>(g.f_hi + r0, f0h);
+        g2_load<NF>(g.f_mid + r0, f0m);
+        g2_load<NF>(g.f_lo + r0, f0l);
         ff b[NF][ND];
 #pragma unroll
         for (int c = 0; c < NF; ++c)
@@ -159,17 +171,13 @@ __global__ __launch_bounds__(128, MG_G2_RHS_MINB) void k_g2_rhs(const __grid_con
             g2_sep(g, h0, l0, s, d);
             if (!g2_basis<DIM>(d, hinv, g.weighted, a, wa)) continue;
             const int64_t rs = (int64_t)s * g.nfp + g.c0;
+            float fh[NF], fm[NF], fl[NF];
+            g2_load<NF>(g.f_hi + rs, fh);
+            g2_load<NF>(g.f_mid + rs, fm);
+            g2_load<NF>(g.f_lo + rs, fl);
 #pragma unroll
-            for (int c = 0; c < NF; c += 4) {
-                const float4 vh = __ldg(reinterpret_cast<const float4 *>(g.f_hi + rs + c));
-                const float4 vm = __ldg(reinterpret_cast<const float4 *>(g.f_mid + rs + c));
-                const float4 vl = __ldg(reinterpret_cast<const float4 *>(g.f_lo + rs + c));
-                const float fh[4] = {vh.x, vh.y, vh.z, vh.w}, fm[4] = {vm.x, vm.y, vm.z, vm.w},
-                            fl[4] = {vl.x, vl.y, vl.z, vl.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    g2_rhs_add<DIM>(b[c + u], wa, ff_diff3(fh[u], fm[u], fl[u], f0h[c + u], f0m[c + u], f0l[c + u]));
-            }
+            for (int c = 0; c < NF; ++c)
+                g2_rhs_add<DIM>(b[c], wa, ff_diff3(fh[c], fm[c], fl[c], f0h[c], f0m[c], f0l[c]));
         }
         const int ncomp = min(NF, g.nf - g.c0);
         const int64_t orow = g.out_rows ? (int64_t)g.out_rows[q] : q;
@@ -459,9 +467,15 @@ extern "C" size_t mg_grad2_solve_workspace_bytes(int64_t nq) {
 
 template <int DIM>
 static int launch_rhs(G2Args g, cudaStream_t st) {
-    for (int c0 = 0; c0 < g.nf; c0 += kG2NF) {
-        g.c0 = c0;
-        k_g2_rhs<DIM, kG2NF><<<(unsigned)((g.nq + 127) / 128), 128, 0, st>>>(g);
+    const unsigned blocks = (unsigned)((g.nq + 127) / 128);
+    for (g.c0 = 0; g.c0 < g.nf; g.c0 += 4) {
+        const int rem = g.nf - g.c0;
+        if (rem >= 3)
+            k_g2_rhs<DIM, 4><<<blocks, 128, 0, st>>>(g);
+        else if (rem == 2)
+            k_g2_rhs<DIM, 2><<<blocks, 128, 0, st>>>(g);
+        else
+            k_g2_rhs<DIM, 1><<<blocks, 128, 0, st>>>(g);
         MG_CHECK_LAUNCH();
     }
     // rows queued by the moments pass, then rows whose solution was not finite
