@@ -211,6 +211,11 @@ int mg_knn_set_persistent_passes(int32_t enabled);
  * means unit masses; density / vol may be NULL. */
 int mg_density(const int32_t *out_rows, const float *hsml, const float *hsml_lo, int64_t nq, const double *m_rows,
                int32_t des_ngb, int32_t dim, double *h_out, double *density, double *vol, void *stream);
+/* The same with the inverse map: row r takes query queries_of_rows[r] (NULL: r).
+ * For all particles in slot order that is mg_cells.rank. */
+int mg_density_rows(const int32_t *queries_of_rows, const float *hsml, const float *hsml_lo, int64_t nq,
+                    const double *m_rows, int32_t des_ngb, int32_t dim, double *h_out, double *density,
+                    double *vol, void *stream);
 /* Smoothing lengths from given neighbour distances (HsmlIter,
  * src/meshoid/kernel_density.py:15-56, without a neighbour search): d2 holds
  * nq rows of k squared distances (FP32, any order, self included as 0);

@@ -27,6 +27,7 @@
 #include "mg_common.cuh"
 #include "mg_grad2.cuh"
 #include "mg_refine.cuh"
+#include "mg_split.cuh"
 
 namespace mg {
 
@@ -83,7 +84,7 @@ __device__ __forceinline__ ff g2_hinv(const G2Args &g, int64_t q) {
 }
 
 template <int DIM>
-__global__ __launch_bounds__(128) void k_g2_moments(const __grid_constant__ G2Args g) {
+__global__ __launch_bounds__(128, 2) void k_g2_moments(const __grid_constant__ G2Args g) {
     constexpr int ND = G2<DIM>::ND, NM = G2<DIM>::NM;
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= g.nq) return;
@@ -365,20 +366,25 @@ __global__ __launch_bounds__(128) void k_hsml_polish(const __grid_constant__ G2A
 }
 
 // f (particle order, FP64) -> slot order three-plane split hi + mid + lo
-__global__ void k_load_fields3(const double *__restrict__ f, const int32_t *__restrict__ order, int64_t n, int nf,
-                               int nfp, float *__restrict__ hi, float *__restrict__ mid, float *__restrict__ lo) {
+// Four components per thread; the split by integer arithmetic (mg_split.cuh).
+__global__ __launch_bounds__(256) void k_load_fields3(const double *__restrict__ f, const int32_t *__restrict__ order,
+                                                      int64_t n, int nf, int nfp, float *__restrict__ hi,
+                                                      float *__restrict__ mid, float *__restrict__ lo) {
     const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= n * nfp) return;
-    const int64_t s = idx / nfp;
-    const int c = (int)(idx - s * nfp);
-    double v = 0.0;
-    if (c < nf) v = f[(int64_t)order[s] * nf + c];
-    const float h = (float)v;
-    const double r = v - (double)h;
-    const float m = (float)r;
-    hi[idx] = h;
-    mid[idx] = m;
-    lo[idx] = (float)(r - (double)m);
+    const int ng = nfp >> 2;
+    if (idx >= n * ng) return;
+    const int64_t s = n * ng <= 0xffffffffll ? (int64_t)((uint32_t)idx / (uint32_t)ng) : idx / ng;
+    const int c = 4 * (int)(idx - s * ng);
+    const double *row = f + (int64_t)order[s] * nf + c;
+    float h[4], m[4], l[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        h[u] = m[u] = l[u] = 0.0f;
+        if (c + u < nf) split3_f64(row[u], h[u], m[u], l[u]);
+    }
+    *reinterpret_cast<float4 *>(hi + 4 * idx) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4 *>(mid + 4 * idx) = make_float4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<float4 *>(lo + 4 * idx) = make_float4(l[0], l[1], l[2], l[3]);
 }
 
 }  // namespace mg
@@ -547,7 +553,7 @@ extern "C" int mg_load_fields3(const mg_cells *c, const double *f, int32_t nf, f
                                void *stream_) {
     if (!c || !f || !hi || !mid || !lo || nf < 1) return MG_ERR_ARG;
     const int nfp = (nf + 3) & ~3;
-    const int64_t tot = c->n * nfp;
+    const int64_t tot = c->n * (nfp / 4);
     k_load_fields3<<<(unsigned)((tot + 255) / 256), 256, 0, as_stream(stream_)>>>(f, c->order, c->n, nf, nfp, hi, mid,
                                                                                   lo);
     MG_CHECK_LAUNCH();

@@ -19,14 +19,30 @@ constexpr int kRsPasses = (64 - kSortLowBit + 7) / 8;  // 7 passes of 8 bits
 
 __global__ void k_bbox_partial(const double *__restrict__ pos, int64_t n, int dim,
                                double *__restrict__ partial) {
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    // compared by their bits as integers (FP64 comparisons run at 1/64 of the FP32
+    // rate): with a negative value's lower bits flipped they order alike; NaN skipped
+    auto ordered = [](long long b) -> long long { return b ^ (b >> 63 & 0x7fffffffffffffffll); };
+    long long lob[3], hib[3];
+    for (int a = 0; a < 3; ++a) {
+        lob[a] = ordered(__double_as_longlong(1e300));
+        hib[a] = ordered(__double_as_longlong(-1e300));
+    }
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        for (int a = 0; a < dim; ++a) {
-            double v = pos[i * dim + a];
-            lo[a] = fmin(lo[a], v);
-            hi[a] = fmax(hi[a], v);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (a >= dim) break;
+            const long long b = __double_as_longlong(pos[i * dim + a]);
+            if ((b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) continue;
+            const long long k = ordered(b);
+            lob[a] = min(lob[a], k);
+            hib[a] = max(hib[a], k);
         }
+    }
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = __longlong_as_double(ordered(lob[a]));
+        hi[a] = __longlong_as_double(ordered(hib[a]));
     }
     __shared__ double s[6][256];
     for (int a = 0; a < 3; ++a) {
@@ -106,9 +122,8 @@ __global__ void k_keys(const double *__restrict__ pos, int64_t n, int dim,
     const double scale = f.inv_side * (double)(1u << kKeyBits);
     uint32_t c[3] = {0, 0, 0};
     for (int a = 0; a < dim; ++a) {
-        double t = (pos[i * dim + a] - o[a]) * scale;
-        t = fmin(fmax(t, 0.0), (double)((1u << kKeyBits) - 1));
-        c[a] = (uint32_t)t;
+        // the conversion saturates (below 0 and NaN to 0): the clamp needs no FP64
+        c[a] = min(__double2uint_rz((pos[i * dim + a] - o[a]) * scale), (1u << kKeyBits) - 1u);
     }
     keys[i] = morton3(c[0], c[1], c[2]);
     vals[i] = (int32_t)i;

@@ -3361,10 +3361,13 @@ __global__ void k_density(const int32_t *__restrict__ out_rows, const float *__r
                           const float *__restrict__ hsml_lo, int64_t nq,
                           const double *__restrict__ m_rows, double des_ngb, double inv_ngb, int dim,
                           double volnorm, double *__restrict__ h_out, double *__restrict__ density,
-                          double *__restrict__ vol) {
-    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (q >= nq) return;
-    const int64_t r = out_rows ? (int64_t)out_rows[q] : q;
+                          double *__restrict__ vol, bool gather) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nq) return;
+    // scatter: query i to row out_rows[i]; gather: row i from query out_rows[i] (the
+    // 4-byte h are read at random instead of 24 bytes of results written so)
+    const int64_t j = out_rows ? (int64_t)out_rows[i] : i;
+    const int64_t q = gather ? j : i, r = gather ? i : j;
     const double h = (double)hsml[q] + (hsml_lo ? (double)hsml_lo[q] : 0.0);
     const double hd = dim == 3 ? h * h * h : (dim == 2 ? h * h : h);
     const double m = m_rows ? m_rows[r] : 1.0;
@@ -3747,18 +3750,30 @@ extern "C" int mg_seed_features(const mg_cells *c, const int32_t *queries, int64
     return MG_OK;
 }
 
-extern "C" int mg_density(const int32_t *out_rows, const float *hsml, const float *hsml_lo, int64_t nq,
-                          const double *m_rows, int32_t des_ngb, int32_t dim, double *h_out, double *density,
-                          double *vol, void *stream_) {
+static int density_rows(const int32_t *rows, bool gather, const float *hsml, const float *hsml_lo, int64_t nq,
+                        const double *m_rows, int32_t des_ngb, int32_t dim, double *h_out, double *density,
+                        double *vol, void *stream_) {
     if (nq <= 0 || !hsml || !h_out || dim < 1 || dim > 3 || des_ngb < 1) return MG_ERR_ARG;
     const double pi = 3.14159265358979323846;
     const double volnorm = dim == 1 ? 2.0 : (dim == 2 ? pi : 4.0 * pi / 3.0);
-    k_density<<<(unsigned)((nq + 255) / 256), 256, 0, as_stream(stream_)>>>(out_rows, hsml, hsml_lo, nq, m_rows,
+    k_density<<<(unsigned)((nq + 255) / 256), 256, 0, as_stream(stream_)>>>(rows, hsml, hsml_lo, nq, m_rows,
                                                                            (double)des_ngb, 1.0 / (double)des_ngb,
                                                                            dim, volnorm, h_out,
-                                                                           density, vol);
+                                                                           density, vol, gather);
     MG_CHECK_LAUNCH();
     return MG_OK;
+}
+
+extern "C" int mg_density(const int32_t *out_rows, const float *hsml, const float *hsml_lo, int64_t nq,
+                          const double *m_rows, int32_t des_ngb, int32_t dim, double *h_out, double *density,
+                          double *vol, void *stream_) {
+    return density_rows(out_rows, false, hsml, hsml_lo, nq, m_rows, des_ngb, dim, h_out, density, vol, stream_);
+}
+
+extern "C" int mg_density_rows(const int32_t *queries_of_rows, const float *hsml, const float *hsml_lo, int64_t nq,
+                               const double *m_rows, int32_t des_ngb, int32_t dim, double *h_out, double *density,
+                               double *vol, void *stream_) {
+    return density_rows(queries_of_rows, true, hsml, hsml_lo, nq, m_rows, des_ngb, dim, h_out, density, vol, stream_);
 }
 
 extern "C" int mg_neighbor_lists(const mg_cells *c, const int32_t *queries, int64_t nq,

@@ -376,9 +376,11 @@ class Meshoid:
         self.density = torch.empty(nq, dtype=torch.float64, device=self.device)
         self.vol = torch.empty(nq, dtype=torch.float64, device=self.device)
         mq = self._m_full if self._full_mask else self._m_full[self.particle_mask].contiguous()
-        check(lib.mg_density(ptr(self._out_rows), ptr(hsml), ptr(hsml_lo), nq, ptr(mq), k, self.dim, ptr(h),
-                             ptr(self.density),
-                             ptr(self.vol), _stream()), "mg_density")
+        # all particles: gathered by slot, so that the results are written in order
+        density, rows = (lib.mg_density_rows, self._rank) if self._queries is None else \
+            (lib.mg_density, self._out_rows)
+        check(density(ptr(rows), ptr(hsml), ptr(hsml_lo), nq, ptr(mq), k, self.dim, ptr(h), ptr(self.density),
+                      ptr(self.vol), _stream()), "mg_density")
         self.kernel_radius = h
 
     def reset_dweights(self):
