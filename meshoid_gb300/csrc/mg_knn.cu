@@ -1773,7 +1773,7 @@ __global__ __launch_bounds__(kKnnWarps * 32, kKnnMinBlocks) void k_knn_hsml(cons
 // find them (a quarter), the selection (a fifth).
 constexpr int kGroupWarps = 2;      // warps per block (independent of each other)
 constexpr int kGroupRuns = 128;     // runs of slots per warp
-constexpr int kGroupStream = 4096;  // particles a warp streams at most (12 bits)
+constexpr int kGroupStream = 4096;  // particles a warp streams at most (12 bits; 13: no faster)
 // Listed candidates per query: 16.5 KB per warp, 14 warps per SM.  88 and 104
 // entries: 3% and 4% slower on 2^22 Plummer particles (more queries left to the
 // warp path; fewer warps); lists cut back to their k nearest when full instead:
@@ -3027,13 +3027,14 @@ __device__ __forceinline__ ff dist_ff(const float4 &h0, const float4 &l0, const 
                                       bool periodic, float box_hi, float box_lo) {
     const float bh[3] = {hb.x, hb.y, hb.z}, bl[3] = {lb.x, lb.y, lb.z};
     const float ah[3] = {h0.x, h0.y, h0.z}, al[3] = {l0.x, l0.y, l0.z};
-    ff r2 = ff{0.0f, 0.0f};
+    ff r2;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
         float l;
         const float d = periodic ? wrap1_ff(bh[c], ah[c], bl[c], al[c], box_hi, box_lo, l)
                                  : sep1_ff(bh[c], ah[c], bl[c], al[c], l);
-        r2 = ff_add(r2, ff_sqr(ff{d, l}));
+        const ff s = ff_sqr(ff{d, l});
+        r2 = c == 0 ? s : ff_add(r2, s);
     }
     return ff_sqrt(r2);
 }
