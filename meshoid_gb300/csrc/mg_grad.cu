@@ -395,7 +395,7 @@ __global__ __launch_bounds__(128) void k_grad(GradArgs g) {
 // of a neighbour's row, 8 lines per warp load where one lane per query reads 32,
 // and the geometry is not repeated for the next components.  Fewer groups than
 // lanes (the last pass) leave several lanes on one group, which then split the
-// neighbours and add their compensated sums.
+// neighbours and add their compensated sums up by halves.
 //
 // Every right-hand side is summed with Kahan compensation (see k_grad).
 //
@@ -471,17 +471,15 @@ __device__ __forceinline__ bool g1_solve(const float L[DIM * (DIM + 1) / 2], con
     return eb * eb > 1e-5f * 1e-5f * nb;
 }
 
-// Compensated sums (r with the negated compensation nc) of the lanes o, 2 o, ..
-// up to four: error-free, the rounding joining the compensation.
-__device__ __forceinline__ void g1_merge(float &r, float &nc, int o) {
-#pragma unroll
-    for (; o < 4; o <<= 1) {
-        const float ro = __shfl_xor_sync(0xffffffffu, r, o), no = __shfl_xor_sync(0xffffffffu, nc, o);
-        float t, e;
-        two_sum(r, ro, t, e);
-        r = t;
-        nc = (nc + no) + e;
-    }
+// Sum of two lanes' compensated sums, r with the negated compensation nc: (give,
+// ngive) goes to the lane o away, whose own joins (r, nc); error-free, the
+// rounding joining the compensation.
+__device__ __forceinline__ void g1_merge(float &r, float &nc, float give, float ngive, int o) {
+    const float ro = __shfl_xor_sync(0xffffffffu, give, o), no = __shfl_xor_sync(0xffffffffu, ngive, o);
+    float t, e;
+    two_sum(r, ro, t, e);
+    r = t;
+    nc = (nc + no) + e;
 }
 
 constexpr int kG1Queries = 32;  // queries per block of 128
@@ -539,37 +537,66 @@ __device__ __forceinline__ bool g1_fields(const GradArgs &g, const G1Smem &S, in
             }
         }
     }
-    float b[4][DIM];
+    // The lanes of a group add their partial sums up by halves: each keeps the
+    // components it will solve, 4 / SUBS of them (component sub of every SUBS),
+    // and gives the others away.
+    constexpr int NC = 4 / SUBS;
+    float r[4][DIM], nc[4][DIM];
 #pragma unroll
     for (int m = 0; m < DIM; ++m)
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            float r[2] = {f2_low(rhs[m][u]), f2_high(rhs[m][u])}, nc[2] = {f2_low(ncmp[m][u]), f2_high(ncmp[m][u])};
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (SUBS > 1) g1_merge(r[e], nc[e], WD);
-                b[2 * u + e][m] = SUBS > 1 ? r[e] + nc[e] : r[e];
-            }
+        for (int u = 0; u < 4; ++u) {
+            r[u][m] = u & 1 ? f2_high(rhs[m][u / 2]) : f2_low(rhs[m][u / 2]);
+            nc[u][m] = u & 1 ? f2_high(ncmp[m][u / 2]) : f2_low(ncmp[m][u / 2]);
         }
+    if constexpr (SUBS == 4) {  // components 0, 1 or 2, 3, with the lane two away
+        const bool up = sub & 2;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 2; ++u) {
 #pragma unroll
-        for (int o = WD; o < 4; o <<= 1) cabs[u] += __shfl_xor_sync(0xffffffffu, cabs[u], o);
-    // solve, test, store: the lanes of a group take its components in turn
+            for (int m = 0; m < DIM; ++m) {
+                const float give = up ? r[u][m] : r[u + 2][m], ngive = up ? nc[u][m] : nc[u + 2][m];
+                r[u][m] = up ? r[u + 2][m] : r[u][m];
+                nc[u][m] = up ? nc[u + 2][m] : nc[u][m];
+                g1_merge(r[u][m], nc[u][m], give, ngive, 2);
+            }
+            const float give = up ? cabs[u] : cabs[u + 2], keep = up ? cabs[u + 2] : cabs[u];
+            cabs[u] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        }
+    }
+    if constexpr (SUBS >= 2) {  // of each two, one
+        const bool up = sub & 1;
+#pragma unroll
+        for (int u = 0; u < NC; ++u) {
+#pragma unroll
+            for (int m = 0; m < DIM; ++m) {
+                const float give = up ? r[2 * u][m] : r[2 * u + 1][m], ngive = up ? nc[2 * u][m] : nc[2 * u + 1][m];
+                r[u][m] = up ? r[2 * u + 1][m] : r[2 * u][m];
+                nc[u][m] = up ? nc[2 * u + 1][m] : nc[2 * u][m];
+                g1_merge(r[u][m], nc[u][m], give, ngive, WD);
+            }
+            const float give = up ? cabs[2 * u] : cabs[2 * u + 1], keep = up ? cabs[2 * u + 1] : cabs[2 * u];
+            cabs[u] = keep + __shfl_xor_sync(0xffffffffu, give, WD);
+        }
+    }
+    // solve, test, store
     bool flag = false;
-    float out[4][DIM];
+    float out[NC][DIM];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        if (SUBS > 1 && u % SUBS != sub) continue;
-        const bool here = mine && c0 + u < g.nf;
-        const bool f = g1_solve<DIM>(L, b[u], cabs[u], cond, hinv, out[u]);
+    for (int u = 0; u < NC; ++u) {
+        const int c = c0 + SUBS * u + sub;
+        float b[DIM];
+#pragma unroll
+        for (int m = 0; m < DIM; ++m) b[m] = SUBS > 1 ? r[u][m] + nc[u][m] : r[u][m];
+        const bool here = mine && c < g.nf;
+        const bool f = g1_solve<DIM>(L, b, cabs[u], cond, hinv, out[u]);
         flag |= here && f;
-        float *o1 = g.d1 + (orow * g.nf + c0 + u) * DIM;
+        float *o1 = g.d1 + (orow * g.nf + c) * DIM;
 #pragma unroll
         for (int m = 0; m < DIM; ++m)  // (whole groups of a 3-D row are stored below)
             if (here && (SUBS > 1 || DIM != 3 || !g.vec_d1)) o1[m] = out[u][m];
     }
-    if (SUBS == 1 && DIM == 3 && g.vec_d1 && mine) {
+    if constexpr (SUBS == 1 && DIM == 3) if (g.vec_d1 && mine) {
         float4 *o = reinterpret_cast<float4 *>(g.d1 + (orow * g.nf + c0) * 3);  // 48 bytes, 16-byte aligned
         o[0] = make_float4(out[0][0], out[0][1 % DIM], out[0][2 % DIM], out[1][0]);
         o[1] = make_float4(out[1][1 % DIM], out[1][2 % DIM], out[2][0], out[2][1 % DIM]);
