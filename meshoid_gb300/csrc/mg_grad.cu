@@ -94,6 +94,21 @@ struct GradArgs {
 
 // cholesky, chol_solve and cond_estimate: mg_chol.cuh
 
+// NF = 4 or 8 components of a neighbour: one load of 16 or 32 bytes (the sweep is
+// bound by the L1 wavefronts of its gathers, and a 32-byte row read by halves
+// costs two: 2^22 Plummer particles, 5 components 1.94 -> 1.77 ms).
+template <int NF>
+__device__ __forceinline__ void grad_load(const float *__restrict__ p, float (&v)[NF]) {
+    if constexpr (NF == 8) {
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+            : "l"(p));
+    } else {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+}
+
 template <int DIM, int ORDER, int NF, bool REFINE = false>
 __global__ __launch_bounds__(128) void k_grad(GradArgs g) {
     static_assert(!REFINE || ORDER == 2, "the refinement step is for order 2");
@@ -169,11 +184,15 @@ __global__ __launch_bounds__(128) void k_grad(GradArgs g) {
             for (int jj = 0; jj <= i; ++jj) M[i * (i + 1) / 2 + jj] += wa[i] * a[jj];
         const float *rh = g.f_hi + (int64_t)s * g.nfp + g.c0;
         const float *rl = g.f_lo ? g.f_lo + (int64_t)s * g.nfp + g.c0 : nullptr;
+        float fh[NF], fl[NF];
+        grad_load<NF>(rh, fh);
+#pragma unroll
+        for (int c = 0; c < NF; ++c) fl[c] = 0.0f;
+        if (rl) grad_load<NF>(rl, fl);
 #pragma unroll
         for (int c = 0; c < NF; c += 4) {
-            const float4 vh = __ldg(reinterpret_cast<const float4 *>(rh + c));
-            float4 vl = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (rl) vl = __ldg(reinterpret_cast<const float4 *>(rl + c));
+            const float4 vh = make_float4(fh[c], fh[c + 1], fh[c + 2], fh[c + 3]),
+                         vl = make_float4(fl[c], fl[c + 1], fl[c + 2], fl[c + 3]);
             const float df[4] = {(vh.x - f0h[c]) + (vl.x - f0l[c]), (vh.y - f0h[c + 1]) + (vl.y - f0l[c + 1]),
                                  (vh.z - f0h[c + 2]) + (vl.z - f0l[c + 2]),
                                  (vh.w - f0h[c + 3]) + (vl.w - f0l[c + 3])};
@@ -1032,8 +1051,8 @@ static int launch_grad(const GradArgs &g0, cudaStream_t st) {
         g.vec_d1 = (g.nf & 3) == 0 && ((uintptr_t)g.d1 & 15) == 0;
         if (g.nfp == 4) {
             k_grad<DIM, ORDER, 4><<<blocks, 128, 0, st>>>(g);
-        } else if (g.nfp == 8) {
-            k_grad<DIM, ORDER, 8><<<blocks, 128, 0, st>>>(g);
+        } else if (g.nfp == 8 && (((uintptr_t)g.f_hi | (uintptr_t)g.f_lo) & 31) == 0) {
+            k_grad<DIM, ORDER, 8><<<blocks, 128, 0, st>>>(g);  // 32-byte rows
         } else {
             const size_t smem = (size_t)g.k * kG1Queries * (sizeof(float4) + sizeof(int32_t));
             MG_CUDA(cudaFuncSetAttribute(k_grad1<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
