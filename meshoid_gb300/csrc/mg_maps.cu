@@ -298,7 +298,7 @@ __global__ void k_sd_items(SdArgs a, int64_t ntiles) {
 // tile of one item stores its pixels, the chunks of a split tile add theirs
 // atomically into the zeroed grid.  The next pair's record is loaded while this
 // one is added.  Bound: instruction issue (~25 per 32 pixels).  2^20 Plummer
-// particles, 1024^2 pixels: 1.02 -> 0.74 ms; 65,536 uniform points, 256^2 pixels
+// particles, 1024^2 pixels: 1.02 -> 0.69 ms; 65,536 uniform points, 256^2 pixels
 // (with the smaller items): 0.40 -> 0.08 ms.
 __global__ __launch_bounds__(32 * kSdWarps) void k_sd_tile(SdArgs a, int64_t ntiles) {
     __shared__ float acc[kSdWarps][kTile * (kTile + 1)];
@@ -340,21 +340,25 @@ __global__ __launch_bounds__(32 * kSdWarps) void k_sd_tile(SdArgs a, int64_t nti
         const float coef2 = 2.0f * (r.coef * kKernel2dNorm);
         // pixel t of the footprint's part of the tile (w x hgt <= 32 x 32):
         // row t / hgt by an FP32 reciprocal, exact for t < 2^10 ((t + 1/2) /
-        // hgt is at least 1/(2 hgt) from an integer); offsets from the
-        // footprint's first node as exact small floats; |d| by r^2 rsqrt(r^2)
-        const float h2 = r.h * r.h, hf = (float)hgt, inv = 1.0f / hf;
-        const float fx0 = (float)(x0 - r.gx0), fy0 = (float)(y0 - r.gy0);
+        // hgt is at least 1/(2 hgt) from an integer); q = |d| / h by q^2 rsqrt(q^2)
+        const float hf = (float)hgt, inv = 1.0f / hf;
+        // in units of h
+        const float s = dxf * hinv;
+        const float ux0 = fmaf(-(float)(x0 - r.gx0), s, r.rx * hinv), uy0 = fmaf(-(float)(y0 - r.gy0), s, r.ry * hinv);
         float *accf = own + (x0 - px0) * (kTile + 1) + (y0 - py0);
         const int skew = kTile + 1 - hgt;
         for (int t = lane; t < w * hgt; t += 32) {
             const float tf = (float)t;
             const float rf = floorf((tf + 0.5f) * inv);
             const float cf = fmaf(-rf, hf, tf);
-            const float ddx = fmaf(-(fx0 + rf), dxf, r.rx);
-            const float ddy = fmaf(-(fy0 + cf), dxf, r.ry);
-            const float r2 = fmaf(ddx, ddx, ddy * ddy);
-            if (r2 > h2) continue;
-            accf[t + (int)rf * skew] += spline_w_half(r2 * rsqrtf(fmaxf(r2, 1e-30f)) * hinv) * coef2;
+            const float ux = fmaf(-rf, s, ux0), uy = fmaf(-cf, s, uy0);
+            const float q2 = fmaf(ux, ux, uy * uy);
+            if (q2 > 1.0f) continue;
+            const float q = q2 * rsqrtf(fmaxf(q2, 1e-30f));
+            // half the spline
+            const float a1 = fmaxf(1.0f - q, 0.0f);
+            const float w = q <= 0.5f ? fmaf(q2, fmaf(3.0f, q, -3.0f), 0.5f) : a1 * a1 * a1;
+            accf[t + (int)rf * skew] += w * coef2;
         }
         __syncwarp();  // the next pair's lanes read what these wrote
     }
@@ -526,33 +530,37 @@ __global__ void k_sd_big_items(SdArgs a, int64_t ntiles) {
 
 // Large footprints, per tile from its own pair list: the work items (a tile's
 // pairs in chunks of kSdBigChunk) are taken by a persistent grid; each CTA
-// stages 256 records at a time in shared memory (1/h and the normalised
-// coefficient computed once per record) and every thread adds their
-// contributions to its 4 pixels in registers.  Each warp owns a 16 x 8
-// sub-block of the tile (lane l: column l % 8, rows l / 8 + 4 j) and skips
-// the records whose footprint box misses it or whose circle misses its nodes
-// by more than 1e-4 of h^2 (there every pixel would evaluate q > 1, a weight
-// of exactly 0): a footprint of 3 x 3 tiles covers about half of its tiles'
-// pixels, so whole sub-blocks drop out.  Per pixel: the offset from the
-// footprint's first node in FP32 exactly as the small path forms it
-// ((gx - gx0) dx with the integer difference converted exactly), |d| by
-// r^2 rsqrt(r^2), and half the spline against twice the coefficient
-// (spline_w_half), 0 beyond q = 1.  No per-pixel box test: the footprint box
+// stages 256 records at a time in shared memory (1/h, the normalised coefficient
+// and the sub-blocks that it reaches, computed once per record) and every thread
+// adds their contributions to its 4 pixels in registers.  Each warp owns a
+// 16 x 8 sub-block of the tile (lane l: column l % 8, rows l / 8 + 4 j) and skips,
+// for each 8 x 8 half, the records whose footprint box misses it or whose circle
+// misses its nodes by more than 1e-4 of h^2 (there every pixel would evaluate
+// q > 1, a weight of exactly 0): a footprint of 3 x 3 tiles covers about half of
+// its tiles' pixels, so whole sub-blocks drop out.  The tests are made by the
+// threads that stage the records, all sub-blocks of one record each; made by
+// each warp for every record they took a third of the kernel.  Per pixel: the offset from the
+// particle in units of h (one FMA from the sub-block's first node, whose
+// integer distance from the footprint's first node is exact), q by
+// q^2 rsqrt(q^2), and half the spline against twice the coefficient, 0 beyond
+// q = 1.  No per-pixel box test: the footprint box
 // holds every node within h of the particle along each axis (the
 // truncations of footprint()), so a node outside it lies at q >= 1 and
 // weighs exactly 0, up to the FP32 rounding of q near 1 (a weight below
 // 1e-18 of the peak; tests/native/sd_cull_check.cu).  The pixels go two to a
-// packed instruction (each half rounds as before: the same bits): 2^20 Plummer
-// particles, 1024^2 pixels 1.50 -> 1.43 ms, bound by the FP32 pipe.  A tile of one item adds its values to the pixels
-// k_sd_tile wrote; the items of a split tile add theirs with FP64 atomics.
+// packed instruction.  2^20 Plummer particles, 1024^2 pixels: 1.50 -> 1.00 ms, of
+// which 0.39 by the shared tests and halves.  A tile of one item adds its values
+// to the pixels k_sd_tile wrote; the items of a split tile add theirs with FP64
+// atomics.
 __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles) {
     __shared__ float4 sa[256];  // rx, ry, 1/h, 2 coef * norm
     __shared__ float4 sb[256];  // gx0, gx1 - gx0, gy0, gy1 - gy0 (exact small integers)
+    __shared__ uint16_t sm[256];  // bits 2 w, 2 w + 1: the halves of warp w's sub-block that take the record
     if (!sd_pairs(a)) return;
     const uint32_t nitems = a.bitem_off[ntiles];
     const int tid = threadIdx.x;
     const float dxf = (float)a.dx;
-    const unsigned long long mdx = f2_pack(-dxf), three = f2_pack(3.0f), mthree = f2_pack(-3.0f),
+    const unsigned long long three = f2_pack(3.0f), mthree = f2_pack(-3.0f),
                              half = f2_pack(0.5f), one = f2_pack(1.0f);
     const double scale = a.conservative ? 1.0 / (a.dx * a.dx) : 1.0;
     for (uint32_t item = blockIdx.x; item < nitems; item += gridDim.x) {
@@ -570,9 +578,9 @@ __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles)
         const int tx = tile / a.ntx, ty = tile % a.ntx;
         const int bx0 = tx * kTile + 16 * ((tid >> 5) & 1), by0 = ty * kTile + 8 * (tid >> 6);  // the warp's sub-block
         const int gy = by0 + (tid & 7), gxb = bx0 + ((tid >> 3) & 3);
-        const float fgy = (float)gy, fbx0 = (float)bx0, fby0 = (float)by0;
-        const unsigned long long fgx[2] = {f2_pack((float)gxb, (float)(gxb + 4)),
-                                           f2_pack((float)(gxb + 8), (float)(gxb + 12))};
+        const float fgy = (float)gy, fbx0 = (float)bx0;
+        const unsigned long long col[2] = {f2_pack((float)(gxb - bx0), (float)(gxb - bx0 + 4)),
+                                           f2_pack((float)(gxb - bx0 + 8), (float)(gxb - bx0 + 12))};
         const uint32_t p0 = a.btile[tile] + j * (uint32_t)kSdBigChunk;
         const uint32_t p1 = min(a.btile[tile + 1], p0 + (uint32_t)kSdBigChunk);
         unsigned long long acc2[2] = {0ull, 0ull};
@@ -580,28 +588,44 @@ __global__ __launch_bounds__(256) void k_sd_tile_pairs(SdArgs a, int64_t ntiles)
             __syncthreads();  // the previous batch is consumed
             if (c0 + tid < p1) {
                 const SdParticle r = a.rec[a.bpairs[c0 + tid]];
-                sa[tid] = make_float4(r.rx, r.ry, 1.0f / r.h, 2.0f * (r.coef * kKernel2dNorm));
-                sb[tid] = make_float4((float)r.gx0, (float)(r.gx1 - r.gx0), (float)r.gy0, (float)(r.gy1 - r.gy0));
+                const float4 pa = make_float4(r.rx, r.ry, 1.0f / r.h, 2.0f * (r.coef * kKernel2dNorm));
+                const float4 pb = make_float4((float)r.gx0, (float)(r.gx1 - r.gx0), (float)r.gy0,
+                                              (float)(r.gy1 - r.gy0));
+                unsigned take = 0;
+#pragma unroll
+                for (int w = 0; w < 16; ++w)
+                    if (!sd_block_skips((float)(tx * kTile + 16 * (w >> 1 & 1) + 8 * (w & 1)),
+                                        (float)(ty * kTile + 8 * (w >> 2)), pa, pb, dxf, 7.0f))
+                        take |= 1u << w;
+                sa[tid] = pa;
+                sb[tid] = pb;
+                sm[tid] = (uint16_t)take;
+            } else {
+                sm[tid] = 0;
             }
             __syncthreads();
-            const int m = (int)min(256u, p1 - c0);
-            for (int e = 0; e < m; ++e) {
+            for (int e0 = 0; e0 < 256 && c0 + e0 < p1; e0 += 32)
+            for (unsigned todo = __ballot_sync(0xffffffffu, sm[e0 + (tid & 31)] >> 2 * (tid >> 5) & 3u); todo;
+                 todo &= todo - 1) {
+                const int e = e0 + __ffs(todo) - 1;
+                const unsigned take = sm[e] >> 2 * (tid >> 5) & 3u;  // warp-uniform
                 const float4 pa = sa[e], pb = sb[e];
-                if (sd_block_skips(fbx0, fby0, pa, pb, dxf)) continue;  // warp-uniform
-                const float oy = fgy - pb.z;  // exact: gy - gy0
-                const float ddy = fmaf(-oy, dxf, pa.y);
-                const unsigned long long ddy2 = f2_pack(ddy * ddy), rx = f2_pack(pa.x), hinv = f2_pack(pa.z),
-                                         coef = f2_pack(pa.w), gx0 = f2_pack(pb.x);
+                // in units of h; the offset of the sub-block's first node from the
+                // footprint's is an exact small integer
+                const float s = dxf * pa.z;
+                const float ux0 = fmaf(-(fbx0 - pb.x), s, pa.x * pa.z), uy = fmaf(-(fgy - pb.z), s, pa.y * pa.z);
+                const unsigned long long uy2 = f2_pack(uy * uy), ux0p = f2_pack(ux0), ms = f2_pack(-s),
+                                         coef = f2_pack(pa.w);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const unsigned long long ox = f2_sub(fgx[u], gx0);  // exact: gx - gx0
-                    const unsigned long long ddx = f2_fma(ox, mdx, rx);
-                    const unsigned long long r2 = f2_fma(ddx, ddx, ddy2);
-                    const unsigned long long rs = f2_pack(rsqrtf(fmaxf(f2_low(r2), 1e-30f)),
-                                                          rsqrtf(fmaxf(f2_high(r2), 1e-30f)));
-                    const unsigned long long q = f2_mul(f2_mul(r2, rs), hinv);
-                    // spline_w_half of both
-                    const unsigned long long in = f2_fma(f2_mul(q, q), f2_fma(three, q, mthree), half);
+                    if (!(take >> u & 1u)) continue;
+                    const unsigned long long ux = f2_fma(col[u], ms, ux0p);
+                    const unsigned long long q2 = f2_fma(ux, ux, uy2);
+                    const unsigned long long rs = f2_pack(rsqrtf(fmaxf(f2_low(q2), 1e-30f)),
+                                                          rsqrtf(fmaxf(f2_high(q2), 1e-30f)));
+                    const unsigned long long q = f2_mul(q2, rs);
+                    // half the spline: 1/2 + q^2 (3 q - 3), and (1 - q)+^3 beyond 1/2
+                    const unsigned long long in = f2_fma(q2, f2_fma(three, q, mthree), half);
                     const unsigned long long c = f2_sub(one, q);
                     const unsigned long long am = f2_pack(fmaxf(f2_low(c), 0.0f), fmaxf(f2_high(c), 0.0f));
                     const unsigned long long out = f2_mul(f2_mul(am, am), am);
