@@ -131,60 +131,119 @@ __global__ void k_keys(const double *__restrict__ pos, int64_t n, int dim,
 
 // ---- LSD radix sort (stable), 8-bit digits ------------------------------------
 
+// Lanes whose digit equals this one's, for a valid lane: eight votes.  With
+// __match_any_sync k_radix_scatter takes 36 us instead of 31 for 2^22 pairs, and the
+// count of the digits 25 us instead of 7.5 with a shared add per key.
+__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = d >> b & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? m : ~m;
+    }
+    return peers;
+}
+
 __global__ __launch_bounds__(kRsThreads) void k_radix_hist(const uint64_t *__restrict__ kin,
                                                            int64_t n, int shift,
                                                            uint32_t *__restrict__ counts, int nb) {
     __shared__ uint32_t h[256];
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     h[tid] = 0;
     __syncthreads();
     const int64_t t0 = (int64_t)blockIdx.x * kRsTile;
+    uint64_t key[kRsRounds];
+#pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
-        int64_t i = t0 + r * kRsThreads + tid;
-        uint32_t d = i < n ? (uint32_t)((kin[i] >> shift) & 255u) : 256u;
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        if (d < 256u && lane == __ffs(peers) - 1) atomicAdd(&h[d], (uint32_t)__popc(peers));
+        const int64_t i = t0 + r * kRsThreads + tid;
+        key[r] = i < n ? kin[i] : 0ull;
+    }
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r) {
+        const int64_t i = t0 + r * kRsThreads + tid;
+        if (i < n) atomicAdd(&h[(uint32_t)((key[r] >> shift) & 255u)], 1u);
     }
     __syncthreads();
     counts[(int64_t)tid * nb + blockIdx.x] = h[tid];
 }
 
+// A block's tile is ordered by digit in shared memory first and written out from
+// there, so that neighbouring threads write neighbouring places: each warp ranks
+// its 256 pairs by itself, one round of 32 after another, and the warps' counts are
+// then scanned digit by digit.  2^22 pairs: 47 -> 31 us, of the 15 us their bytes
+// take; a round of 256 at a time, written straight to its place, took four barriers
+// a round and a sector a pair.
 __global__ __launch_bounds__(kRsThreads) void k_radix_scatter(
     const uint64_t *__restrict__ kin, const int32_t *__restrict__ vin, uint64_t *__restrict__ kout,
     int32_t *__restrict__ vout, int64_t n, int shift, const uint32_t *__restrict__ offsets, int nb) {
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t wcnt[kRsThreads / 32][256];
+    constexpr int kWarps = kRsThreads / 32;
+    __shared__ uint64_t skey[kRsTile];
+    __shared__ int32_t sval[kRsTile];
+    __shared__ uint32_t wcnt[kWarps][256];  // per warp and digit: count, then first place in the tile
+    __shared__ uint32_t to[256];            // place in the output less the place in the tile
+    __shared__ uint32_t wsum[kWarps];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    base[tid] = offsets[(int64_t)tid * nb + blockIdx.x];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) wcnt[w][tid] = 0;
     const int64_t t0 = (int64_t)blockIdx.x * kRsTile;
+    const int64_t i0 = t0 + warp * (32 * kRsRounds) + lane;
+    uint64_t key[kRsRounds];
+    uint32_t rank[kRsRounds];
+    int32_t val[kRsRounds];
+#pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
+        const int64_t i = i0 + 32 * r;
+        key[r] = i < n ? kin[i] : 0ull;
+        val[r] = i < n ? vin[i] : 0;
+    }
+    const uint32_t first = offsets[(int64_t)tid * nb + blockIdx.x];  // of digit tid
+    __syncthreads();
 #pragma unroll
-        for (int w = 0; w < kRsThreads / 32; ++w) wcnt[w][tid] = 0;
-        __syncthreads();
-        const int64_t i = t0 + r * kRsThreads + tid;
-        const bool valid = i < n;
-        uint64_t key = valid ? kin[i] : 0ull;
-        int32_t val = valid ? vin[i] : 0;
-        uint32_t d = valid ? (uint32_t)((key >> shift) & 255u) : 256u;
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        int rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = (uint32_t)__popc(peers);
-        __syncthreads();
-        uint32_t run = base[tid];
+    for (int r = 0; r < kRsRounds; ++r) {
+        const bool valid = i0 + 32 * r < n;
+        const uint32_t d = (uint32_t)((key[r] >> shift) & 255u);
+        const unsigned peers = digit_peers(d, valid);
+        const uint32_t before = valid ? wcnt[warp][d] : 0u;
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = before + (uint32_t)__popc(peers);
+        rank[r] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+    }
+    __syncthreads();
+    // digit tid: its pairs in the tile, and in the warps before each
+    uint32_t run = 0;
 #pragma unroll
-        for (int w = 0; w < kRsThreads / 32; ++w) {
-            uint32_t c = wcnt[w][tid];
-            wcnt[w][tid] = run;
-            run += c;
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t c = wcnt[w][tid];
+        wcnt[w][tid] = run;
+        run += c;
+    }
+    const uint32_t inc = (uint32_t)warp_incl_scan((int)run);
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    uint32_t start = inc - run;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) start += w < warp ? wsum[w] : 0u;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) wcnt[w][tid] += start;
+    to[tid] = first - start;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r) {
+        if (i0 + 32 * r < n) {
+            const uint32_t at = wcnt[warp][(uint32_t)((key[r] >> shift) & 255u)] + rank[r];
+            skey[at] = key[r];
+            sval[at] = val[r];
         }
-        base[tid] = run;
-        __syncthreads();
-        if (valid) {
-            uint32_t p = wcnt[warp][d] + (uint32_t)rank;
-            kout[p] = key;
-            vout[p] = val;
-        }
-        __syncthreads();
+    }
+    __syncthreads();
+    const int m = (int)min((int64_t)kRsTile, n - t0);
+    for (int i = tid; i < m; i += kRsThreads) {
+        const uint64_t k = skey[i];
+        const uint32_t p = to[(uint32_t)((k >> shift) & 255u)] + (uint32_t)i;
+        kout[p] = k;
+        vout[p] = sval[i];
     }
 }
 
@@ -221,9 +280,10 @@ __global__ __launch_bounds__(1024) void k_radix_one(const uint64_t *__restrict__
         __syncthreads();  // the pass before has written its pairs
         for (int c = i0; c < i1; c += 32) {
             const int i = c + lane;
-            const uint32_t d = i < i1 ? (uint32_t)((S.key[from][i] >> shift) & 255u) : 256u;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
-            if (d < 256u && lane == __ffs(peers) - 1) S.cnt[warp][d] += (uint16_t)__popc(peers);
+            const bool valid = i < i1;
+            const uint32_t d = valid ? (uint32_t)((S.key[from][i] >> shift) & 255u) : 0u;
+            const unsigned peers = digit_peers(d, valid);
+            if (valid && lane == __ffs(peers) - 1) S.cnt[warp][d] += (uint16_t)__popc(peers);
             __syncwarp();
         }
         __syncthreads();
@@ -252,8 +312,8 @@ __global__ __launch_bounds__(1024) void k_radix_one(const uint64_t *__restrict__
             const int i = c + lane;
             const bool valid = i < i1;
             const uint64_t key = valid ? S.key[from][i] : 0ull;
-            const uint32_t d = valid ? (uint32_t)((key >> shift) & 255u) : 256u;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t d = (uint32_t)((key >> shift) & 255u);
+            const unsigned peers = digit_peers(d, valid);
             const uint32_t base = valid ? S.cnt[warp][d] : 0u;
             __syncwarp();
             if (valid) {
@@ -313,8 +373,11 @@ __global__ void k_cell_count(const uint64_t *__restrict__ keys, int64_t n, int s
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     uint64_t c = i < n ? (keys[i] >> shift) : ~0ull;
-    unsigned peers = __match_any_sync(0xffffffffu, c);
-    if (i < n && lane == __ffs(peers) - 1) atomicAdd(&count[c], (uint32_t)__popc(peers));
+    // sorted keys: a cell's particles are neighbouring lanes
+    const uint64_t before = __shfl_up_sync(0xffffffffu, c, 1);
+    const bool head = lane == 0 || c != before;
+    const unsigned after = __ballot_sync(0xffffffffu, head) >> lane >> 1;  // heads above this lane
+    if (head && i < n) atomicAdd(&count[c], (uint32_t)(after ? __ffs(after) : 32 - lane));
 }
 
 // ---- bricks: refinement tables below the dense level ----------------------------
