@@ -16,6 +16,7 @@
 #include "mg_common.cuh"
 #include "mg_cube.cuh"
 #include "mg_scan.cuh"
+#include "mg_split.cuh"
 
 namespace mg {
 
@@ -72,26 +73,37 @@ struct GdRange {
     float u[3], s;
 };
 
+// v rounded to FP32, without the FP64 pipe where the exponent allows.
+__device__ __forceinline__ float gd_round32(double v) {
+    float f, unit;
+    int32_t rem;
+    return split_f64(v, f, rem, unit) ? f : (float)v;
+}
+
 // Node range of particle p (the reference's truncation, clipped without a box).
 // The truncations of (x - h) / dx + 1 and (x + h) / dx are decided in FP32
 // from the FP32 roundings of x and h (each within ~4e-7 (|x| + h) / dx of
 // the FP64 quotients); where either lies within 1e-6 (|x| + h) / dx + 1e-6
-// of an integer the FP64 division decides, as in the reference.  FP64
-// divisions and conversions run at a small fraction of the FP32 rate on
-// this GPU, and this set-up ran twice per particle with ten of them.
+// of an integer the FP64 division decides, as in the reference.  FP64 runs at
+// 1/64 of the FP32 rate on this GPU and the pass that only counts was bound by
+// it: x is formed with two additions instead of the reference's three (the same
+// but for the last bit, which the FP64 decision forms as the reference does),
+// rounded by its bits, and the offset u (U) is left out where it is not used.
+template <bool U>
 __device__ __forceinline__ bool gd_range(const double *__restrict__ pos, const double *__restrict__ h, int64_t p,
                                          const double ctr[3], double size, double dx, double inv_dx, int res,
                                          bool periodic, GdRange &g) {
-    const double hs = h[p];
-    const float hf = (float)hs, invf = (float)inv_dx;
+    const double hs = h[p], shift = size / 2 - dx / 2;
+    const float hf = gd_round32(hs), invf = (float)inv_dx;
     bool empty = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double xs = pos[p * 3 + d] - ctr[d] + size / 2 - dx / 2;
+        const double off = pos[p * 3 + d] - ctr[d], xs = off + shift;
         int a, b;
-        if (!trunc_pair32((float)xs, hf, invf, a, b)) {
-            a = (int)((xs - hs) / dx + 1);
-            b = (int)((xs + hs) / dx);
+        if (!trunc_pair32(gd_round32(xs), hf, invf, a, b)) {
+            const double xr = off + size / 2 - dx / 2;
+            a = (int)((xr - hs) / dx + 1);
+            b = (int)((xr + hs) / dx);
         }
         if (!periodic) {
             a = max(a, 0);
@@ -100,9 +112,9 @@ __device__ __forceinline__ bool gd_range(const double *__restrict__ pos, const d
         g.lo[d] = a;
         g.cnt[d] = b - a + 1;
         empty = empty || g.cnt[d] <= 0;
-        g.u[d] = (float)(xs * inv_dx - (double)a);
+        if (U) g.u[d] = gd_round32(xs * inv_dx - (double)a);
     }
-    g.s = (float)dx / hf;
+    if (U) g.s = (float)dx / hf;
     return !empty;
 }
 
@@ -118,17 +130,20 @@ __device__ __forceinline__ uint32_t gd_tiles(const GdRange &g) {
     return t;
 }
 
-// count != 0: only the number of tile overlaps (an upper bound of the pairs),
-// summed into *npairs.  Otherwise: normalisation, direct deposit of wrapping
-// cubes, per-particle data of the rest and their overlap counts.
+// COUNT: only the number of tile overlaps (an upper bound of the pairs), summed
+// into *npairs.  Otherwise: normalisation, direct deposit of wrapping cubes,
+// per-particle data of the rest and their overlap counts.  2^21 Plummer particles,
+// 128^3 nodes: 780 -> 510 us (with a nest of three loops per lane 7,400
+// instructions per 32 particles), and 123 -> 66 us the count, by its FP64.
+template <bool COUNT>
 __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__restrict__ pos,
                                                            const double *__restrict__ h,
                                                            const double *__restrict__ f, int64_t n, double cx,
                                                            double cy, double cz, double size, int res, bool periodic,
-                                                           bool count, unsigned long long *__restrict__ npairs,
+                                                           unsigned long long *__restrict__ npairs,
                                                            uint32_t *__restrict__ tcount, float4 *__restrict__ pu,
                                                            int4 *__restrict__ plo, int4 *__restrict__ pcnt,
-                                                           double *__restrict__ pfac, double *__restrict__ grid,
+                                                           double *__restrict__ grid,
                                                            int64_t *__restrict__ n_skipped) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * kDepWarps;
@@ -140,14 +155,51 @@ __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__rest
         // lane: FP64 set-up of particle p0 + lane
         const int64_t pl = p0 + lane;
         GdRange gr;
-        const bool anyl = pl < n && gd_range(pos, h, pl, ctr, size, dx, inv_dx, res, periodic, gr);
+        const bool anyl = pl < n && gd_range<!COUNT>(pos, h, pl, ctr, size, dx, inv_dx, res, periodic, gr);
         const bool insidel = anyl && gd_inside(gr, res);
-        if (count) {
+        if (COUNT) {
             if (insidel) counted += gd_tiles(gr);
             continue;
         }
+        // A lane normalises its own particle when the cube is small (the
+        // usual case: ~30 nodes at 128^3 over a Plummer sphere); the warp
+        // takes the large cubes and those that wrap around the box one
+        // particle after another (a chain of shuffles, loop and reduction
+        // per particle, too serial for the small ones).  One loop over the
+        // nodes, not a nest: lanes with cubes of different shapes would each
+        // wait for the longest of the others in every level of it.
+        const int64_t totl = insidel ? (int64_t)gr.cnt[0] * gr.cnt[1] * gr.cnt[2] : 0;
+        const bool own = insidel && totl <= kGdOwnNodes;
+        float wsl = 0.0f;  // sum of the particle's weights
+        if (own) {
+            const int tot = (int)totl, n1 = gr.cnt[1], n2 = gr.cnt[2];
+            const float s = gr.s;
+            float fi = 0.0f, fj = 0.0f, fl = 0.0f;
+            int j = 0, l = 0;
+            float a = gr.u[0] * s, b = gr.u[1] * s, ab = fmaf(b, b, a * a);
+            for (int c = 0; c < tot; ++c) {
+                const float z = (gr.u[2] - fl) * s;
+                wsl += spline_w(sqrtf(fmaf(z, z, ab)));
+                fl += 1.0f;
+                if (++l == n2) {
+                    l = 0;
+                    fl = 0.0f;
+                    fj += 1.0f;
+                    if (++j == n1) {
+                        j = 0;
+                        fj = 0.0f;
+                        fi += 1.0f;
+                        a = (gr.u[0] - fi) * s;
+                    }
+                    b = (gr.u[1] - fj) * s;
+                    ab = fmaf(b, b, a * a);
+                }
+            }
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, anyl && !own);
+        const unsigned insm = __ballot_sync(0xffffffffu, insidel);
         NodeCube gl;
-        if (anyl) {
+        if (todo) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 gl.lo[d] = gr.lo[d];
@@ -156,32 +208,8 @@ __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__rest
                 gl.s[d] = gr.s;
             }
         }
-        const unsigned anym = __ballot_sync(0xffffffffu, anyl), insm = __ballot_sync(0xffffffffu, insidel);
-        uint32_t my_tiles = 0;
-        // A lane normalises its own particle when the cube is small (the
-        // usual case: ~30 nodes at 128^3 over a Plummer sphere); the warp
-        // takes the large cubes and those that wrap around the box one
-        // particle after another (a chain of shuffles, loop and reduction
-        // per particle, too serial for the small ones).
-        bool own = false;
-        if (insidel && (int64_t)gr.cnt[0] * gr.cnt[1] * gr.cnt[2] <= kGdOwnNodes) {
-            own = true;
-            const float s3[3] = {gr.s, gr.s, gr.s};
-            float ws = 0.0f;
-            for (int i = 0; i < gr.cnt[0]; ++i)
-                for (int jj = 0; jj < gr.cnt[1]; ++jj)
-                    for (int l = 0; l < gr.cnt[2]; ++l) ws += cube_w(gr.u, s3, i, jj, l);
-            if (ws > 0.0f) {
-                my_tiles = gd_tiles(gr);
-                pu[pl] = make_float4(gr.u[0], gr.u[1], gr.u[2], gr.s);
-                plo[pl] = make_int4(gr.lo[0], gr.lo[1], gr.lo[2], 0);
-                pcnt[pl] = make_int4(gr.cnt[0], gr.cnt[1], gr.cnt[2], 0);
-                pfac[pl] = f[pl] / (double)ws * inv_vol;
-            }
-        }
-        const unsigned ownm = __ballot_sync(0xffffffffu, own);
-        for (int k = 0; k < 32; ++k) {
-            if (!(anym >> k & 1u) || (ownm >> k & 1u)) continue;
+        for (; todo; todo &= todo - 1) {
+            const int k = __ffs(todo) - 1;
             const int64_t p = p0 + k;
             const NodeCube g = shfl_cube(gl, k);
             const bool inside = insm >> k & 1u;
@@ -200,35 +228,41 @@ __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__rest
                 wsum += cube_w(g.u, g.s, i, j, l);
             }
             wsum = warp_sum(wsum);
+            if (inside) {
+                if (lane == k) wsl = wsum;
+                continue;
+            }
             if (!(wsum > 0.0f)) continue;
             // one lane divides (a warp-wide FP64 division is 32 of them, and
             // FP64 runs at a small fraction of the FP32 rate on this GPU)
             double fac = 0.0;
             if (lane == 0) fac = f[p] / (double)wsum * inv_vol;
             fac = __shfl_sync(0xffffffffu, fac, 0);
-            if (inside) {
-                if (lane == k) {
-                    my_tiles = gd_tiles(gr);
-                    pu[p] = make_float4(gr.u[0], gr.u[1], gr.u[2], gr.s);
-                    plo[p] = make_int4(gr.lo[0], gr.lo[1], gr.lo[2], 0);
-                    pcnt[p] = make_int4(gr.cnt[0], gr.cnt[1], gr.cnt[2], 0);
-                    pfac[p] = fac;
-                }
-            } else {
-                for (int64_t c = lane; c < total; c += 32) {
-                    int i, j, l;
-                    cube_node(c, cd, i, j, l);
-                    const float w = cube_w(g.u, g.s, i, j, l);
-                    if (w == 0.0f) continue;
-                    const int gx = pmod(g.lo[0] + i, res), gy = pmod(g.lo[1] + j, res), gz = pmod(g.lo[2] + l, res);
-                    atomicAdd(grid + ((int64_t)gx * res + gy) * res + gz, fac * (double)w);
-                }
+            for (int64_t c = lane; c < total; c += 32) {
+                int i, j, l;
+                cube_node(c, cd, i, j, l);
+                const float w = cube_w(g.u, g.s, i, j, l);
+                if (w == 0.0f) continue;
+                const int gx = pmod(g.lo[0] + i, res), gy = pmod(g.lo[1] + j, res), gz = pmod(g.lo[2] + l, res);
+                atomicAdd(grid + ((int64_t)gx * res + gy) * res + gz, fac * (double)w);
             }
+        }
+        // the tiles take the factor in FP32: one division and one rounding per
+        // particle, here
+        uint32_t my_tiles = 0;
+        if (insidel && wsl > 0.0f) {
+            my_tiles = gd_tiles(gr);
+            const float fac = (float)(f[pl] / (double)wsl * inv_vol);
+            pu[pl] = make_float4(gr.u[0], gr.u[1], gr.u[2], gr.s);
+            plo[pl] = make_int4(gr.lo[0], gr.lo[1], gr.lo[2], __float_as_int(fac));
+            pcnt[pl] = make_int4(gr.cnt[0], gr.cnt[1], gr.cnt[2], 0);
         }
         if (pl < n) tcount[pl] = my_tiles;
     }
-    counted = warp_sum(counted);
-    if (count && lane == 0 && counted) atomicAdd(npairs, counted);
+    if (COUNT) {
+        counted = warp_sum(counted);
+        if (lane == 0 && counted) atomicAdd(npairs, counted);
+    }
 }
 
 // overlaps of particle p at [toff[p], toff[p + 1]) (none: deposited directly or nothing)
@@ -278,8 +312,7 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
                                                           const uint32_t *__restrict__ nitems,
                                                           const int32_t *__restrict__ val,
                                                           const float4 *__restrict__ pu, const int4 *__restrict__ plo,
-                                                          const int4 *__restrict__ pcnt,
-                                                          const double *__restrict__ pfac, int res,
+                                                          const int4 *__restrict__ pcnt, int res,
                                                           double *__restrict__ grid) {
     __shared__ float acc[kGdTile * kGdTile * kGdTile];
     const int item = blockIdx.x;
@@ -296,7 +329,7 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
         const float4 u4 = pu[p];
         const int4 lo = plo[p], cn = pcnt[p];
         const float u[3] = {u4.x, u4.y, u4.z}, s3[3] = {u4.w, u4.w, u4.w};
-        const float fac = (float)pfac[p];
+        const float fac = __int_as_float(lo.w);
         // the cube's nodes inside this tile
         const int a0 = max(lo.x, base[0]), b0 = min(lo.x + cn.x, base[0] + kGdTile);
         const int a1 = max(lo.y, base[1]), b1 = min(lo.y + cn.y, base[1] + kGdTile);
@@ -476,9 +509,9 @@ extern "C" int mg_grid_density_count(const double *pos, const double *h, int64_t
     cudaStream_t st = as_stream(stream_);
     MG_CUDA(cudaMemsetAsync(npairs, 0, sizeof(int64_t), st));
     if (n == 0) return MG_OK;
-    k_gd_prep<<<dep_blocks(n), kDepWarps * 32, 0, st>>>(pos, h, nullptr, n, cx, cy, cz, size, res, periodic != 0, true,
-                                                       reinterpret_cast<unsigned long long *>(npairs), nullptr, nullptr,
-                                                       nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_gd_prep<true><<<dep_blocks(n), kDepWarps * 32, 0, st>>>(
+        pos, h, nullptr, n, cx, cy, cz, size, res, periodic != 0, reinterpret_cast<unsigned long long *>(npairs),
+        nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     MG_CHECK_LAUNCH();
     return MG_OK;
 }
@@ -494,7 +527,7 @@ extern "C" size_t mg_grid_density_workspace_bytes(int64_t n, int64_t npairs, int
     const int64_t maxit = (int64_t)nt + npairs / kGdChunk + 1;
     return align_up(sizeof(uint32_t) * (size_t)(n + 1)) + align_up(scan_workspace_bytes(n + 1)) +
            align_up(sizeof(float4) * (size_t)(n + 1)) + 2 * align_up(sizeof(int4) * (size_t)(n + 1)) +
-           align_up(sizeof(double) * (size_t)(n + 1)) + align_up(sizeof(uint64_t) * (size_t)(npairs + 1)) +
+           align_up(sizeof(uint64_t) * (size_t)(npairs + 1)) +
            align_up(sizeof(int32_t) * (size_t)(npairs + 1)) + radix_sort_workspace_bytes(npairs + 1) +
            3 * align_up(sizeof(uint32_t) * (size_t)(nt + 2)) + align_up(scan_workspace_bytes(nt + 1)) +
            align_up(sizeof(int4) * (size_t)maxit) + 4096;
@@ -520,7 +553,6 @@ extern "C" int mg_grid_density(const double *pos, const double *h, const double 
     float4 *pu = w.take<float4>((size_t)n + 1);
     int4 *plo = w.take<int4>((size_t)n + 1);
     int4 *pcnt = w.take<int4>((size_t)n + 1);
-    double *pfac = w.take<double>((size_t)n + 1);
     uint64_t *key = w.take<uint64_t>((size_t)npairs + 1);
     int32_t *val = w.take<int32_t>((size_t)npairs + 1);
     void *sort_ws = w.take<char>(radix_sort_workspace_bytes(npairs + 1));
@@ -531,8 +563,8 @@ extern "C" int mg_grid_density(const double *pos, const double *h, const double 
     int4 *items = w.take<int4>((size_t)maxit);
     if (!w.ok()) return MG_ERR_ARG;
     // 1. normalisation, direct deposits of wrapping cubes, overlap counts
-    k_gd_prep<<<dep_blocks(n), kDepWarps * 32, 0, st>>>(pos, h, f, n, cx, cy, cz, size, res, periodic != 0, false,
-                                                       nullptr, tcount, pu, plo, pcnt, pfac, grid, n_skipped);
+    k_gd_prep<false><<<dep_blocks(n), kDepWarps * 32, 0, st>>>(pos, h, f, n, cx, cy, cz, size, res, periodic != 0,
+                                                              nullptr, tcount, pu, plo, pcnt, grid, n_skipped);
     MG_CHECK_LAUNCH();
     MG_CUDA(cudaMemsetAsync(tcount + n, 0, sizeof(uint32_t), st));
     int rc = exclusive_scan_u32(tcount, tcount, n + 1, scan_ws, st);  // -> offsets
@@ -559,7 +591,7 @@ extern "C" int mg_grid_density(const double *pos, const double *h, const double 
     k_gd_items<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(tbeg, ioff, nt, items);
     MG_CHECK_LAUNCH();
     // 4. shared-memory accumulation per item, one global add per node
-    k_gd_tile<<<(unsigned)maxit, kGdWarps * 32, 0, st>>>(items, nitems, val, pu, plo, pcnt, pfac, res, grid);
+    k_gd_tile<<<(unsigned)maxit, kGdWarps * 32, 0, st>>>(items, nitems, val, pu, plo, pcnt, res, grid);
     MG_CHECK_LAUNCH();
     return MG_OK;
 }
