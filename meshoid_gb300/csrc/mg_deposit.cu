@@ -133,7 +133,7 @@ __device__ __forceinline__ uint32_t gd_tiles(const GdRange &g) {
 // COUNT: only the number of tile overlaps (an upper bound of the pairs), summed
 // into *npairs.  Otherwise: normalisation, direct deposit of wrapping cubes,
 // per-particle data of the rest and their overlap counts.  2^21 Plummer particles,
-// 128^3 nodes: 780 -> 510 us (with a nest of three loops per lane 7,400
+// 128^3 nodes: 780 -> 460 us (with a nest of three loops per lane 7,400
 // instructions per 32 particles), and 123 -> 66 us the count, by its FP64.
 template <bool COUNT>
 __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__restrict__ pos,
@@ -222,10 +222,18 @@ __global__ __launch_bounds__(kDepWarps * 32) void k_gd_prep(const double *__rest
             const int64_t total = (int64_t)g.cnt[0] * g.cnt[1] * g.cnt[2];
             const CubeDiv cd = cube_div(g.cnt[1], g.cnt[2], total);
             float wsum = 0.0f;
-            for (int64_t c = lane; c < total; c += 32) {
-                int i, j, l;
-                cube_node(c, cd, i, j, l);
-                wsum += cube_w(g.u, g.s, i, j, l);
+            if (cd.small) {
+                for (int c = lane; c < (int)total; c += 32) {
+                    int i, j, l;
+                    cube_node(c, cd, i, j, l);
+                    wsum += cube_w(g.u, g.s, i, j, l);
+                }
+            } else {
+                for (int64_t c = lane; c < total; c += 32) {
+                    int i, j, l;
+                    cube_node(c, cd, i, j, l);
+                    wsum += cube_w(g.u, g.s, i, j, l);
+                }
             }
             wsum = warp_sum(wsum);
             if (inside) {
@@ -308,6 +316,17 @@ __global__ void k_gd_items(const uint32_t *__restrict__ tbeg, const uint32_t *__
     for (uint32_t s = b; s < e; s += kGdChunk, ++it) items[it] = make_int4(t, (int)s, (int)min(e, s + kGdChunk), 0);
 }
 
+// One block per item.  A warp takes up to 32 overlaps at a time: each lane cuts one
+// cube to the tile and leaves it in shared memory, and the lanes then walk the
+// nodes of all of them as one list, 32 at a time, whatever the cubes' sizes (a warp
+// per overlap set every cube up in all its lanes and left half of them idle: ~15
+// nodes of a cube lie in a tile at 128^3 over a Plummer sphere).  Items of few
+// overlaps are spread over the eight warps.  The warps take overlaps in turn and
+// keep step, so that a node's values are added about in the particles' order: FP32
+// sums of up to kGdChunk values, whose roundings follow the order (without the
+// barrier maps of 2^21 particles moved by 2.6e-8, with it by 1.6e-8, and two runs of
+// any form differ by 0.7e-8).  2^21 Plummer particles, 128^3 nodes: 1105 -> 465 us,
+// bound by the instructions of the weights and of the shared-memory adds.
 __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restrict__ items,
                                                           const uint32_t *__restrict__ nitems,
                                                           const int32_t *__restrict__ val,
@@ -315,6 +334,9 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
                                                           const int4 *__restrict__ pcnt, int res,
                                                           double *__restrict__ grid) {
     __shared__ float acc[kGdTile * kGdTile * kGdTile];
+    __shared__ float4 su[kGdWarps][32];  // offset from the lowest node, node spacing / h
+    __shared__ float4 so[kGdWarps][32];  // first node in the tile less the lowest node; factor
+    __shared__ float4 sn[kGdWarps][32];  // 1 / counts of the last two axes; counts and first place; first of the list
     const int item = blockIdx.x;
     if (item >= (int)*nitems) return;
     const int4 it = items[item];
@@ -324,26 +346,52 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
     for (int c = threadIdx.x; c < kGdTile * kGdTile * kGdTile; c += blockDim.x) acc[c] = 0.0f;
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int e = it.y + wib; e < it.z; e += kGdWarps) {
-        const int p = val[e];
-        const float4 u4 = pu[p];
-        const int4 lo = plo[p], cn = pcnt[p];
-        const float u[3] = {u4.x, u4.y, u4.z}, s3[3] = {u4.w, u4.w, u4.w};
-        const float fac = __int_as_float(lo.w);
-        // the cube's nodes inside this tile
-        const int a0 = max(lo.x, base[0]), b0 = min(lo.x + cn.x, base[0] + kGdTile);
-        const int a1 = max(lo.y, base[1]), b1 = min(lo.y + cn.y, base[1] + kGdTile);
-        const int a2 = max(lo.z, base[2]), b2 = min(lo.z + cn.z, base[2] + kGdTile);
-        const int n1 = b1 - a1, n2 = b2 - a2, nn = (b0 - a0) * n1 * n2;
-        const CubeDiv cd = cube_div(n1, n2, nn);
-        for (int c = lane; c < nn; c += 32) {
-            int i, j, l;
-            cube_node(c, cd, i, j, l);
-            const int gx = a0 + i, gy = a1 + j, gz = a2 + l;
-            const float w = cube_w(u, s3, gx - lo.x, gy - lo.y, gz - lo.z);
-            if (w != 0.0f)
-                atomicAdd(&acc[((gx - base[0]) * kGdTile + (gy - base[1])) * kGdTile + (gz - base[2])], fac * w);
+        const int per = min(32, (it.z - it.y + kGdWarps - 1) / kGdWarps);
+    for (int e0 = it.y; e0 < it.z; e0 += kGdWarps * per) {
+        int nn = 0;
+        const int e = e0 + lane * kGdWarps + wib;
+        if (lane < per && e < it.z) {
+            const int p = val[e];
+            const int4 lo = plo[p], cn = pcnt[p];
+            // the cube's nodes inside this tile
+            const int a0 = max(lo.x, base[0]), b0 = min(lo.x + cn.x, base[0] + kGdTile);
+            const int a1 = max(lo.y, base[1]), b1 = min(lo.y + cn.y, base[1] + kGdTile);
+            const int a2 = max(lo.z, base[2]), b2 = min(lo.z + cn.z, base[2] + kGdTile);
+            const int n1 = b1 - a1, n2 = b2 - a2;
+            nn = (b0 - a0) * n1 * n2;
+            const int at = ((a0 - base[0]) * kGdTile + (a1 - base[1])) * kGdTile + (a2 - base[2]);
+            su[wib][lane] = pu[p];
+            so[wib][lane] = make_float4((float)(a0 - lo.x), (float)(a1 - lo.y), (float)(a2 - lo.z),
+                                        __int_as_float(lo.w));
+            sn[wib][lane] = make_float4(1.0f / (float)n1, 1.0f / (float)n2, __int_as_float(n1 | n2 << 8 | at << 16),
+                                        0.0f);
         }
+        const int end = warp_incl_scan(nn), start = end - nn;
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        sn[wib][lane].w = __int_as_float(start);
+        __syncwarp();
+        int before = 0;  // cubes that start ahead of the window
+        for (int w0 = 0; w0 < total; w0 += 32) {
+            const bool here = nn > 0 && (start >> 5) == (w0 >> 5);
+            const unsigned heads = __reduce_or_sync(0xffffffffu, here ? 1u << (start & 31) : 0u);
+            const int k = before + __popc(heads & ((2u << lane) - 1u)) - 1;
+            before += __popc(heads);
+            if (w0 + lane < total) {
+                const float4 u = su[wib][k], o = so[wib][k], nd = sn[wib][k];
+                const int pk = __float_as_int(nd.z), n1 = pk & 255, n2 = pk >> 8 & 255;
+                const int c = w0 + lane - __float_as_int(nd.w);
+                // quotients of small whole numbers, exact (mg_cube.cuh)
+                const int col = (int)(((float)c + 0.5f) * nd.y);
+                const int l = c - col * n2;
+                const int i = (int)(((float)col + 0.5f) * nd.x);
+                const int j = col - i * n1;
+                const float x = (u.x - (o.x + (float)i)) * u.w, y = (u.y - (o.y + (float)j)) * u.w,
+                            z = (u.z - (o.z + (float)l)) * u.w;
+                const float w = spline_w(sqrtf(fmaf(z, z, fmaf(y, y, x * x))));
+                if (w != 0.0f) atomicAdd(&acc[(pk >> 16) + (i * kGdTile + j) * kGdTile + l], o.w * w);
+            }
+        }
+        __syncthreads();  // the next overlaps overwrite these; the warps keep step
     }
     __syncthreads();
     for (int c = threadIdx.x; c < kGdTile * kGdTile * kGdTile; c += blockDim.x) {
