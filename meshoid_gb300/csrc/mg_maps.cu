@@ -298,7 +298,7 @@ __global__ void k_sd_items(SdArgs a, int64_t ntiles) {
 // tile of one item stores its pixels, the chunks of a split tile add theirs
 // atomically into the zeroed grid.  The next pair's record is loaded while this
 // one is added.  Bound: instruction issue (~25 per 32 pixels).  2^20 Plummer
-// particles, 1024^2 pixels: 1.02 -> 0.69 ms; 65,536 uniform points, 256^2 pixels
+// particles, 1024^2 pixels: 1.02 -> 0.74 ms; 65,536 uniform points, 256^2 pixels
 // (with the smaller items): 0.40 -> 0.08 ms.
 __global__ __launch_bounds__(32 * kSdWarps) void k_sd_tile(SdArgs a, int64_t ntiles) {
     __shared__ float acc[kSdWarps][kTile * (kTile + 1)];
@@ -340,25 +340,23 @@ __global__ __launch_bounds__(32 * kSdWarps) void k_sd_tile(SdArgs a, int64_t nti
         const float coef2 = 2.0f * (r.coef * kKernel2dNorm);
         // pixel t of the footprint's part of the tile (w x hgt <= 32 x 32):
         // row t / hgt by an FP32 reciprocal, exact for t < 2^10 ((t + 1/2) /
-        // hgt is at least 1/(2 hgt) from an integer); q = |d| / h by q^2 rsqrt(q^2)
-        const float hf = (float)hgt, inv = 1.0f / hf;
-        // in units of h
-        const float s = dxf * hinv;
-        const float ux0 = fmaf(-(float)(x0 - r.gx0), s, r.rx * hinv), uy0 = fmaf(-(float)(y0 - r.gy0), s, r.ry * hinv);
+        // hgt is at least 1/(2 hgt) from an integer); offsets from the
+        // footprint's first node as exact small floats; |d| by r^2 rsqrt(r^2).
+        // Not in units of h: most h here are the smallest that the map allows, and
+        // the rounding of dx / h would move all those particles the same way.
+        const float h2 = r.h * r.h, hf = (float)hgt, inv = 1.0f / hf;
+        const float fx0 = (float)(x0 - r.gx0), fy0 = (float)(y0 - r.gy0);
         float *accf = own + (x0 - px0) * (kTile + 1) + (y0 - py0);
         const int skew = kTile + 1 - hgt;
         for (int t = lane; t < w * hgt; t += 32) {
             const float tf = (float)t;
             const float rf = floorf((tf + 0.5f) * inv);
             const float cf = fmaf(-rf, hf, tf);
-            const float ux = fmaf(-rf, s, ux0), uy = fmaf(-cf, s, uy0);
-            const float q2 = fmaf(ux, ux, uy * uy);
-            if (q2 > 1.0f) continue;
-            const float q = q2 * rsqrtf(fmaxf(q2, 1e-30f));
-            // half the spline
-            const float a1 = fmaxf(1.0f - q, 0.0f);
-            const float w = q <= 0.5f ? fmaf(q2, fmaf(3.0f, q, -3.0f), 0.5f) : a1 * a1 * a1;
-            accf[t + (int)rf * skew] += w * coef2;
+            const float ddx = fmaf(-(fx0 + rf), dxf, r.rx);
+            const float ddy = fmaf(-(fy0 + cf), dxf, r.ry);
+            const float r2 = fmaf(ddx, ddx, ddy * ddy);
+            if (r2 > h2) continue;
+            accf[t + (int)rf * skew] += spline_w_half(r2 * rsqrtf(fmaxf(r2, 1e-30f)) * hinv) * coef2;
         }
         __syncwarp();  // the next pair's lanes read what these wrote
     }
