@@ -433,6 +433,12 @@ int mg_gradient_weights(const double *pos, int32_t dim, const int64_t *ngb, int3
 size_t mg_kde_1d_workspace_bytes(int64_t ng);
 int mg_kde_1d(const double *x, const double *bw, int64_t n, const double *grid, int64_t ng, double *f,
               void *workspace, size_t workspace_bytes, void *stream);
+/* First-order expansion about a particle, in FP64 (Reconstruct,
+ * src/meshoid/Meshoid.py:425-431): out (nt, nc) = f[nn] + sum_a (targets -
+ * pos[nn])_a grad[row, :, a], separations wrapped to half of boxsize (<= 0: no
+ * box).  f (n, nc), pos (n, dim), targets (nt, dim), grad (rows, nc, dim). */
+int mg_taylor1(const double *f, const double *pos, const int64_t *nn, const int64_t *row, const double *targets,
+               const float *grad, int64_t nt, int32_t nc, int32_t dim, double boxsize, double *out, void *stream);
 /* Nearest particle of each target point (k = 1 query of
  * src/meshoid/Meshoid.py:410): nn (nt) particle indices, ties by index. */
 size_t mg_nn_query_workspace_bytes(int64_t nt);

@@ -148,6 +148,7 @@ SIGNATURES = {
     "mg_batched_workspace_bytes": (c_sz, [ctypes.POINTER(MgSnapshot), c_i32, c_i32]),
     "mg_batched_run": (c_i32, [ctypes.POINTER(MgSnapshot), c_i32, c_i32, c_f32, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "mg_nn_query_workspace_bytes": (c_sz, [c_i64]),
+    "mg_taylor1": (c_i32, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_i64, c_i32, c_i32, c_f64, c_vp, c_vp]),
     "mg_nn_query": (c_i32, [ctypes.POINTER(MgCells), c_vp, c_i64, c_vp, c_vp, c_sz, c_vp]),
 }
 

@@ -779,21 +779,30 @@ class Meshoid:
         nn = self._nn(target_points)
         unique, inv = torch.unique(nn, sorted=True, return_inverse=True)
         f = _dev_tensor(f, torch.float64, self.device)
-        f_t = f[nn].clone()
         if order == 0:
-            return f_t
-        dx = target_points - self.pos[nn]
-        if self.boxsize is not None:
-            b = float(self.boxsize)
-            dx = torch.where(dx.abs() > b / 2, -torch.copysign(b - dx.abs(), dx), dx)
+            return f[nn].clone()
         if not (unique.numel() == self.particle_mask.numel() and bool(torch.equal(unique, self.particle_mask))):
             self.particle_mask = unique
             self._full_mask = False
             self._set_queries()
             self.TreeUpdate()
             self.reset_dweights()
-        grad = self.D(f, order=order)[inv].double()
-        f_t += torch.einsum("ij,i...j->i...", dx, grad)
+        D = self.D(f, order=order)
+        # one pass where nothing is differentiated or broadcast
+        if (order == 1 and target_points.shape == (nn.shape[0], self.dim)
+                and (self.boxsize is None or float(self.boxsize) > 0)
+                and not (f.requires_grad or target_points.requires_grad or self.pos.requires_grad)):
+            f_t = torch.empty((nn.shape[0],) + tuple(f.shape[1:]), dtype=torch.float64, device=self.device)
+            check(self._lib.mg_taylor1(ptr(f), ptr(self.pos), ptr(nn), ptr(inv), ptr(target_points),
+                                       ptr(D), nn.shape[0], f.numel() // self.N, self.dim,
+                                       float(self.boxsize or 0.0), ptr(f_t), _stream()), "mg_taylor1")
+            return f_t
+        f_t = f[nn].clone()
+        dx = target_points - self.pos[nn]
+        if self.boxsize is not None:
+            b = float(self.boxsize)
+            dx = torch.where(dx.abs() > b / 2, -torch.copysign(b - dx.abs(), dx), dx)
+        f_t += torch.einsum("ij,i...j->i...", dx, D[inv].double())
         if order == 1:
             return f_t
         d2f = self.D2(f)[inv].double()
