@@ -65,7 +65,8 @@ __device__ __forceinline__ float cube_w(const float u[3], const float s[3], int 
 // directly with global atomics (few particles: those within h of the faces).
 constexpr int kGdTile = 8;        // nodes per tile side
 constexpr int kGdChunk = 4096;    // overlaps per work item
-constexpr int kGdWarps = 8;       // warps per work-item CTA
+constexpr int kGdWarps = 4;       // warps per work-item CTA
+constexpr int kGdLayers = kGdTile / kGdWarps;  // layers of a tile's nodes per warp
 constexpr int kGdOwnNodes = 64;   // cubes up to this many nodes are normalised by their particle's lane
 
 struct GdRange {
@@ -316,17 +317,18 @@ __global__ void k_gd_items(const uint32_t *__restrict__ tbeg, const uint32_t *__
     for (uint32_t s = b; s < e; s += kGdChunk, ++it) items[it] = make_int4(t, (int)s, (int)min(e, s + kGdChunk), 0);
 }
 
-// One block per item.  A warp takes up to 32 overlaps at a time: each lane cuts one
-// cube to the tile and leaves it in shared memory, and the lanes then walk the
-// nodes of all of them as one list, 32 at a time, whatever the cubes' sizes (a warp
-// per overlap set every cube up in all its lanes and left half of them idle: ~15
-// nodes of a cube lie in a tile at 128^3 over a Plummer sphere).  Items of few
-// overlaps are spread over the eight warps.  The warps take overlaps in turn and
-// keep step, so that a node's values are added about in the particles' order: FP32
-// sums of up to kGdChunk values, whose roundings follow the order (without the
-// barrier maps of 2^21 particles moved by 2.6e-8, with it by 1.6e-8, and two runs of
-// any form differ by 0.7e-8).  2^21 Plummer particles, 128^3 nodes: 1105 -> 465 us,
-// bound by the instructions of the weights and of the shared-memory adds.
+// One block per item, two layers of the tile's nodes per warp.  A warp takes 32
+// overlaps at a time: each lane cuts one cube to the warp's layers and leaves it in
+// shared memory, and the lanes then walk the nodes of all of them as one list, 32 at
+// a time, whatever the cubes' sizes (a warp per overlap set every cube up in all its
+// lanes and left half of them idle: ~15 nodes of a cube lie in a tile at 128^3 over a
+// Plummer sphere).  A node belongs to one warp, which adds its values in the order
+// of the particles: the FP32 sums of up to kGdChunk values are the same in every
+// run.  Shared out by overlaps among eight warps they followed the warps' timing,
+// and the total of a 24^3 deposit of 16,384 particles moved between -0.5e-9 and
+// -1.5e-9 (now always -0.97e-9).  2^21 Plummer particles, 128^3 nodes: 1105 -> 560 us
+// (465 us by overlaps, 630 us with a layer per warp), bound by the instructions of
+// the weights and of the shared-memory adds.
 __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restrict__ items,
                                                           const uint32_t *__restrict__ nitems,
                                                           const int32_t *__restrict__ val,
@@ -346,29 +348,33 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
     for (int c = threadIdx.x; c < kGdTile * kGdTile * kGdTile; c += blockDim.x) acc[c] = 0.0f;
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-        const int per = min(32, (it.z - it.y + kGdWarps - 1) / kGdWarps);
-    for (int e0 = it.y; e0 < it.z; e0 += kGdWarps * per) {
-        int nn = 0;
-        const int e = e0 + lane * kGdWarps + wib;
-        if (lane < per && e < it.z) {
-            const int p = val[e];
-            const int4 lo = plo[p], cn = pcnt[p];
-            // the cube's nodes inside this tile
-            const int a0 = max(lo.x, base[0]), b0 = min(lo.x + cn.x, base[0] + kGdTile);
-            const int a1 = max(lo.y, base[1]), b1 = min(lo.y + cn.y, base[1] + kGdTile);
-            const int a2 = max(lo.z, base[2]), b2 = min(lo.z + cn.z, base[2] + kGdTile);
-            const int n1 = b1 - a1, n2 = b2 - a2;
-            nn = (b0 - a0) * n1 * n2;
-            const int at = ((a0 - base[0]) * kGdTile + (a1 - base[1])) * kGdTile + (a2 - base[2]);
-            su[wib][lane] = pu[p];
-            so[wib][lane] = make_float4((float)(a0 - lo.x), (float)(a1 - lo.y), (float)(a2 - lo.z),
-                                        __int_as_float(lo.w));
-            sn[wib][lane] = make_float4(1.0f / (float)n1, 1.0f / (float)n2, __int_as_float(n1 | n2 << 8 | at << 16),
-                                        0.0f);
+        const int x0 = base[0] + wib * kGdLayers, x1 = x0 + kGdLayers;
+    for (int e0 = it.y; e0 < it.z; e0 += 32) {
+        const int e = e0 + lane;
+        int4 lo = make_int4(0, 0, 0, 0), cn = lo;
+        if (e < it.z) {
+            lo = plo[val[e]];
+            cn = pcnt[val[e]];
+        }
+        // the cube's nodes in this warp's layers of the tile
+        const int a0 = max(lo.x, x0), b0 = min(lo.x + cn.x, x1);
+        const int a1 = max(lo.y, base[1]), b1 = min(lo.y + cn.y, base[1] + kGdTile);
+        const int a2 = max(lo.z, base[2]), b2 = min(lo.z + cn.z, base[2] + kGdTile);
+        const int n1 = b1 - a1, n2 = b2 - a2;
+        const int nn = e < it.z && b0 > a0 ? (b0 - a0) * n1 * n2 : 0;
+        const unsigned some = __ballot_sync(0xffffffffu, nn > 0);
+        const int at = __popc(some & ((1u << lane) - 1u));
+        if (nn > 0) {
+            const int first = ((a0 - base[0]) * kGdTile + (a1 - base[1])) * kGdTile + (a2 - base[2]);
+            su[wib][at] = pu[val[e]];
+            so[wib][at] = make_float4((float)(a0 - lo.x), (float)(a1 - lo.y), (float)(a2 - lo.z),
+                                      __int_as_float(lo.w));
+            sn[wib][at] = make_float4(1.0f / (float)n1, 1.0f / (float)n2, __int_as_float(n1 | n2 << 8 | first << 16),
+                                      0.0f);
         }
         const int end = warp_incl_scan(nn), start = end - nn;
         const int total = __shfl_sync(0xffffffffu, end, 31);
-        sn[wib][lane].w = __int_as_float(start);
+        if (nn > 0) sn[wib][at].w = __int_as_float(start);
         __syncwarp();
         int before = 0;  // cubes that start ahead of the window
         for (int w0 = 0; w0 < total; w0 += 32) {
@@ -391,7 +397,7 @@ __global__ __launch_bounds__(kGdWarps * 32) void k_gd_tile(const int4 *__restric
                 if (w != 0.0f) atomicAdd(&acc[(pk >> 16) + (i * kGdTile + j) * kGdTile + l], o.w * w);
             }
         }
-        __syncthreads();  // the next overlaps overwrite these; the warps keep step
+        __syncwarp();  // the next overlaps overwrite these
     }
     __syncthreads();
     for (int c = threadIdx.x; c < kGdTile * kGdTile * kGdTile; c += blockDim.x) {
