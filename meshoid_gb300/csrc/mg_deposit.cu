@@ -4,8 +4,8 @@
 //   mg_ppz_cube           Grid_PPZ_DataCube      src/meshoid/grid_deposition.py:339-392
 //   mg_weighted_interp3d  WeightedGridInterp3D   src/meshoid/grid_deposition.py:439-531
 //
-// One warp per particle (grid-stride over particles).  The node range of a
-// particle is computed from its FP64 position with the reference's own
+// PPZ and weighted deposits: one warp per particle (grid-stride over particles);
+// GridDensity by tiles of nodes, below.  The node range of a particle is computed from its FP64 position with the reference's own
 // expressions (C truncation, the same clipping or periodic wrap), so every
 // particle touches exactly the reference's nodes.  Kernel weights are FP32:
 // the particle's offset from its lowest node is taken in FP64 in node units
@@ -58,8 +58,8 @@ __device__ __forceinline__ float cube_w(const float u[3], const float s[3], int 
 // GridDensity.  A particle's cube of nodes is usually small (~30 nodes at
 // 128^3 over a Plummer sphere) but millions of them share the central nodes,
 // so one global atomic per node and particle is contention-bound.  Instead
-// each particle's normalisation is found first (warp per particle, no
-// atomics), the (8^3-node tile, particle) overlaps are sorted by tile, and one
+// each particle's normalisation is found first (in its lane, or by the warp
+// for large cubes; no atomics), the (8^3-node tile, particle) overlaps are sorted by tile, and one
 // CTA per chunk of a tile's overlaps accumulates in shared memory and adds
 // each node once.  With a box, a cube that wraps around the grid is deposited
 // directly with global atomics (few particles: those within h of the faces).
