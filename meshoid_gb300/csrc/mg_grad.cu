@@ -946,7 +946,9 @@ __global__ __launch_bounds__(32) void k_grad_fix1(GradArgs g) {
                 double sd = A[j][j];
 #pragma unroll
                 for (int k2 = 0; k2 < j; ++k2) sd -= Lc[j][k2] * Lc[j][k2];
-                spd = spd && sd > 1e-14 * fmax(A[0][0], 1e-300);
+                // a pivot of the size of its diagonal's rounding means fewer
+                // directions than dim inside the kernel, also where A[0][0] is small
+                spd = spd && sd > 1e-14 * fmax(A[0][0], 1e-300) && sd > 1e-13 * A[j][j];
                 const double d = sqrt(spd ? sd : 1.0);
                 Lc[j][j] = d;
                 inv[j] = 1.0 / d;
